@@ -15,6 +15,7 @@ import sys
 HERE = os.path.dirname(os.path.abspath(__file__))
 ROOT = os.path.dirname(HERE)
 SRC = os.path.join(HERE, "csrc", "bls_engine.cu")
+INCLUDES = [os.path.join(HERE, "csrc", "bls_gather.cuh")]
 LIB_DIR = os.path.join(HERE, "lib")
 LIB = os.path.join(LIB_DIR, "libastrotransit_b200.so")
 HEADER = os.path.join(ROOT, "include", "astrotransit_b200.h")
@@ -40,7 +41,7 @@ def needs_build() -> bool:
     if not os.path.exists(LIB):
         return True
     mt = os.path.getmtime(LIB)
-    return any(os.path.getmtime(p) > mt for p in (SRC, HEADER))
+    return any(os.path.getmtime(p) > mt for p in (SRC, HEADER, *INCLUDES))
 
 
 def build(verbose: bool = False, force: bool = False) -> str:

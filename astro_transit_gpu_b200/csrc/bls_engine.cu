@@ -32,10 +32,13 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <climits>
 #include <cstdarg>
 #include <cstdio>
 #include <cstring>
 #include <string>
+#include <type_traits>
+#include <utility>
 #include <vector>
 
 #include "../../include/astrotransit_b200.h"
@@ -86,6 +89,15 @@ constexpr double kDefaultMergeRun = 8.0;   // atb_params.merge_run = 0
 // binned geometry, whose larger histograms want the bigger shared-memory share)
 constexpr int kDefaultFixedThreads = kBlockB;
 constexpr int kChunk = 32 * kR;        // staged points of one warp's fold step
+// cost of one look-up of the prefix-gather search in scattered points (bls_gather.cuh)
+#ifndef ATB_LOOK_COST_BINNED
+#define ATB_LOOK_COST_BINNED 1.1
+#endif
+#ifndef ATB_LOOK_COST_FIXED
+#define ATB_LOOK_COST_FIXED 5.0
+#endif
+constexpr double kLookCostBinned = ATB_LOOK_COST_BINNED;
+constexpr double kLookCostFixed = ATB_LOOK_COST_FIXED;
 constexpr double kMagicSlot = 4503599627370497.0;   // 2^52 + 1: x + C (rz) = 2^52 + int(x) + 1, x in (-1, 2^31 - 1)
 constexpr double kMagicFloor = 6755399441055744.0;  // 1.5*2^52: (m + C)(rd) - C = floor(m), |m| < 2^50
 
@@ -222,11 +234,25 @@ struct SearchArgs {
     unsigned long long* best_key;  // winner-take-all per-curve records (or NULL)
     int tile_p;                    // periods per work-queue tile (1..kTileP)
     double merge_run;              // expected points per bin from which kFoldChunk is used
+    const struct TableStat* tstats;  // per curve, for the gather kernel
+    const int* n_scatter;          // 0: every period is gathered (NULL: none is)
+    unsigned char* scatter;        // per period: 0 when the gather kernel searches it (NULL: none)
+    const long long* flag_off;     // per curve: its first entry of `scatter`
 };
 
 // ----------------------------------------------------------------------------
 // shared device helpers
 // ----------------------------------------------------------------------------
+
+// First period of a work-queue tile of curve c (the lo-th of the queue).  The
+// longest periods of the grid come first: they have the most bins, and at the
+// end of the queue a tile of them would keep one CTA busy alone.
+__device__ __forceinline__ long long tile_start(const SearchArgs& a, long long tile, int lo,
+                                                int c) {
+    const long long n = a.tile_off[lo + 1] - a.tile_off[lo], i = tile - a.tile_off[lo];
+    const double* P = a.periods + a.per_beg[c];
+    return (P[a.per_cnt[c] - 1] > P[0] ? n - 1 - i : i) * a.tile_p;
+}
 
 __device__ __forceinline__ int q_scale(double m, int qbits) {
     if (!(m > 0.0)) return 0;
@@ -710,6 +736,8 @@ __device__ __forceinline__ void team_sync(const Team& tm) {
 struct GroupSmem {
     double tP[kTileP];   // the tile's periods
     int tNB[kTileP];     // and their bin counts
+    int tI[kTileP];      // and their places in the tile
+    int tn;              // how many there are
     double2 PIP[kMaxG];  // (P, 1/P) of each period of the group
     int2 NBB[kMaxG];     // (bin count, histogram offset) of each period
     int fmode[kMaxG];    // fold mode of each period (kFold*)
@@ -725,7 +753,7 @@ struct GroupSmem {
     float den[kMaxWarps];
     int key[kMaxWarps];
     long long tile;
-    long long pb, pe, pn;
+    long long pb, pe;
     int curve;
     int G;
     int total;
@@ -1798,10 +1826,13 @@ __device__ void run_group(const SearchArgs& a, GroupSmem& gs, longlong2* H, cons
     }
 }
 
+#include "bls_gather.cuh"
+
 template <int GEOM, int NT, int MINB>
 __global__ void __launch_bounds__(NT, MINB) search_kernel(const SearchArgs a) {
     extern __shared__ __align__(16) longlong2 s_hist[];
     __shared__ GroupSmem gs;
+    if (a.n_scatter && *a.n_scatter == 0) return;
 
     for (;;) {
         if (threadIdx.x == 0) {
@@ -1815,7 +1846,7 @@ __global__ void __launch_bounds__(NT, MINB) search_kernel(const SearchArgs a) {
                 }
                 const int c = a.order[lo];
                 gs.curve = c;
-                gs.pb = (tile - a.tile_off[lo]) * a.tile_p;
+                gs.pb = tile_start(a, tile, lo, c);
                 gs.pe = min(gs.pb + a.tile_p, a.per_cnt[c]);
             }
         }
@@ -1834,30 +1865,44 @@ __global__ void __launch_bounds__(NT, MINB) search_kernel(const SearchArgs a) {
             gs.dbins[threadIdx.x] = a.dbins[c * kMaxDur + threadIdx.x];
             gs.dur[threadIdx.x] = a.durations[a.dur_beg[c] + threadIdx.x];
         }
-        long long pn = gs.pb;
-        const long long pe = gs.pe;
-        // the tile's periods and bin counts, loaded in parallel
-        for (int i = threadIdx.x; i < (int)(pe - pn); i += NT) {
-            double P = a.periods[pbeg + pn + i];
-            if (!(P > 0.0) || !(P < 1.0e300)) {
-                atomicOr(a.status, 4);
-                P = 1.0;
+        // the tile's periods and bin counts, loaded in parallel, without those the
+        // gather kernel searches
+        const long long p0 = gs.pb;
+        const int np = (int)(gs.pe - p0);
+        for (int i = threadIdx.x; i < np; i += NT) {
+            const bool mine = !a.scatter || a.scatter[a.flag_off[c] + p0 + i] != 0;
+            int at = i;
+            if (a.scatter) {
+                at = 0;
+                for (int k = 0; k < i; ++k) at += a.scatter[a.flag_off[c] + p0 + k] != 0;
+                if (i == np - 1) gs.tn = at + (mine ? 1 : 0);
+            } else if (i == np - 1) {
+                gs.tn = np;
             }
-            gs.tP[i] = P;
-            gs.tNB[i] = (GEOM == ATB_GEOM_BINNED)
-                            ? binned_nbins(P, st.inv_bin_dur, a.oversample, a.max_bins)
-                            : a.n_bins_fixed;
+            if (mine) {
+                double P = a.periods[pbeg + p0 + i];
+                if (!(P > 0.0) || !(P < 1.0e300)) {
+                    atomicOr(a.status, 4);
+                    P = 1.0;
+                }
+                gs.tP[at] = P;
+                gs.tI[at] = i;
+                gs.tNB[at] = (GEOM == ATB_GEOM_BINNED)
+                                 ? binned_nbins(P, st.inv_bin_dur, a.oversample, a.max_bins)
+                                 : a.n_bins_fixed;
+            }
         }
         __syncthreads();
+        const int pe = gs.tn;
+        int pn = 0;
         while (pn < pe) {
             if (threadIdx.x == 0) {
                 int g = 0, base = 0;
-                long long p = pn;
+                int p = pn;
                 double ipmax = 0.0, pmax = 0.0;
                 while (p < pe && g < kMaxG) {
-                    const int li = (int)(p - gs.pb);
-                    const double P = gs.tP[li];
-                    const int NB = gs.tNB[li];
+                    const double P = gs.tP[p];
+                    const int NB = gs.tNB[p];
                     const int need = NB + 2;
                     if (g > 0 && base + need > a.cap) break;
                     const double IP = 1.0 / P;
@@ -1865,7 +1910,7 @@ __global__ void __launch_bounds__(NT, MINB) search_kernel(const SearchArgs a) {
                     pmax = max(pmax, P);
                     gs.PIP[g] = make_double2(P, IP);
                     gs.NBB[g] = make_int2(NB, base);
-                    gs.slot[g] = obeg + p;
+                    gs.slot[g] = obeg + p0 + gs.tI[p];
                     base += need;
                     ++g;
                     ++p;
@@ -2175,8 +2220,21 @@ struct atb_plan {
     StageArgs sa{};
     SearchArgs qa{};
     int* best = nullptr;
+    // device words zeroed before every execution
+    struct Control {
+        unsigned long long tiles;    // search kernel's work counter
+        unsigned long long gathers[2];  // gather kernels' (packed, weighted)
+        int status;
+        int n_gather[2], n_scatter;     // some period is gathered / scattered
+        int nb_max;                  // set-up: the largest bin count
+    };
+    Control* control = nullptr;
     int* status = nullptr;
-    unsigned long long* counter = nullptr;
+    // prefix-gather search (its tables exist when ga.off is set)
+    GatherArgs ga{};
+    TableStat* tstats = nullptr;
+    int gather_grid[2] = {0, 0};  // packed, weighted
+    int gather_smem[2] = {0, 0};
     // plans made by atb_plan_create_async: scratch comes from the stream-ordered
     // allocator and every set-up copy, the status read-back and the release run
     // on `stream`, so that no call waits for other streams' work
@@ -2221,19 +2279,43 @@ int plan_alloc(atb_plan* p, T** out, size_t count) {
     return ATB_OK;
 }
 
-template <typename T>
-int plan_upload(atb_plan* p, T** out, const std::vector<T>& host) {
-    int rc = plan_alloc(p, out, host.size());
-    if (rc) return rc;
-    if (!host.empty()) {
-        // from pageable memory: returns once the data are staged, so `host` may go
-        ATB_CUDA(p->h, p->async ? cudaMemcpyAsync(*out, host.data(), host.size() * sizeof(T),
-                                                  cudaMemcpyHostToDevice, p->stream)
-                                : cudaMemcpy(*out, host.data(), host.size() * sizeof(T),
-                                             cudaMemcpyHostToDevice));
+// A plan's device arrays in one allocation, its host index arrays in one copy: a
+// plan of one curve is made for every call of the per-call API, where each
+// separate allocation and copy costs several microseconds of host time.
+struct PlanArrays {
+    std::vector<std::pair<void**, size_t>> slots;  // pointer to set, byte offset
+    std::vector<char> host;                        // the uploads (they come first)
+    size_t bytes = 0;
+    size_t place(void** out, size_t n) {
+        const size_t at = (bytes + 255) / 256 * 256;
+        slots.push_back({out, at});
+        bytes = at + std::max<size_t>(n, 1);
+        return at;
     }
-    return ATB_OK;
-}
+    template <typename T>
+    void upload(T** out, const std::vector<T>& v) {
+        const size_t at = place(reinterpret_cast<void**>(out), v.size() * sizeof(T));
+        host.resize(at + v.size() * sizeof(T));
+        if (!v.empty()) std::memcpy(host.data() + at, v.data(), v.size() * sizeof(T));
+    }
+    template <typename T>
+    void scratch(T** out, size_t count) {
+        place(reinterpret_cast<void**>(out), count * sizeof(T));
+    }
+    int commit(atb_plan* p) {
+        char* base = nullptr;
+        int rc = plan_alloc(p, &base, bytes);
+        if (rc) return rc;
+        for (auto& s : slots) *s.first = base + s.second;
+        // from pageable memory: returns once the data are staged, so `host` may go
+        if (!host.empty())
+            ATB_CUDA(p->h, p->async ? cudaMemcpyAsync(base, host.data(), host.size(),
+                                                      cudaMemcpyHostToDevice, p->stream)
+                                    : cudaMemcpy(base, host.data(), host.size(),
+                                                 cudaMemcpyHostToDevice));
+        return ATB_OK;
+    }
+};
 
 void plan_free(atb_plan* p) {
     for (void* q : p->allocs) {
@@ -2292,6 +2374,111 @@ int launch_stage(atb_plan* p, cudaStream_t s) {
     else
         stage_kernel<float><<<p->n_curves, kStageBlock, 0, s>>>(p->sa);
     ATB_CUDA(p->h, cudaGetLastError());
+    return ATB_OK;
+}
+
+using GatherFn = void (*)(const SearchArgs, const GatherArgs);
+GatherFn gather_fn(int geom, bool packed) {
+    if (geom == ATB_GEOM_BINNED)
+        return packed ? gather_kernel<ATB_GEOM_BINNED, true> : gather_kernel<ATB_GEOM_BINNED, false>;
+    return packed ? gather_kernel<ATB_GEOM_FIXED, true> : gather_kernel<ATB_GEOM_FIXED, false>;
+}
+
+// The search: gathered periods (when the plan has tables), then scattered ones.
+int launch_search(atb_plan* p, cudaStream_t s) {
+    if (p->ga.tab) {
+        if (p->prm.geometry == ATB_GEOM_BINNED)
+            table_kernel<ATB_GEOM_BINNED><<<p->n_curves, kTableBlock, 0, s>>>(p->qa, p->ga,
+                                                                             p->tstats);
+        else
+            table_kernel<ATB_GEOM_FIXED><<<p->n_curves, kTableBlock, 0, s>>>(p->qa, p->ga,
+                                                                            p->tstats);
+        ATB_CUDA(p->h, cudaGetLastError());
+        for (int w = 0; w < p->ga.vs; ++w) {  // counting curves, then weighted ones
+            gather_fn(p->prm.geometry, w == 0)<<<p->gather_grid[w], kGatherBlock, p->gather_smem[w],
+                                                 s>>>(p->qa, p->ga);
+            ATB_CUDA(p->h, cudaGetLastError());
+        }
+    }
+    search_fn(p->prm.geometry, p->nt)<<<p->grid, p->nt, p->smem_bytes, s>>>(p->qa);
+    ATB_CUDA(p->h, cudaGetLastError());
+    return ATB_OK;
+}
+
+// Tables and launch shape of the gather kernel.  Without memory for the
+// tables the plan scatters every period.
+int plan_gather(atb_plan* p, const std::vector<long long>& pt_off,
+                const std::vector<long long>& per_cnt, bool weighted) {
+    const int nc = p->n_curves;
+    GatherArgs ga{};
+    ga.vs = weighted ? 2 : 1;
+    ga.ring = 384;  // astropy bins: windows of up to 192 bins
+    if (p->prm.geometry == ATB_GEOM_FIXED) {
+        // (entries up to two periods: windows that wrap)
+        ga.ring = (2 * std::min(p->prm.n_bins, 1 << 20) + 2 + 31) / 32 * 32;
+        if (ga.ring > 1024) return ATB_OK;
+    } else if (p->prm.oversample >= kHeadMax) {
+        return ATB_OK;
+    }
+    std::vector<long long> cell_off(nc + 1, 0);
+    for (int c = 0; c < nc; ++c) {
+        // a handful of periods would not repay the table
+        const long long n = per_cnt[c] < kGatherMinPeriods ? 0 : pt_off[c + 1] - pt_off[c];
+        cell_off[c + 1] = cell_off[c] + gather_cells(n);
+    }
+    // A curve's table is made by one CTA; few periods in all finish sooner without
+    // (the table kernel weighs it curve by curve).
+    long long periods = 0;
+    for (int c = 0; c < nc; ++c) periods += per_cnt[c];
+    const size_t cells = (size_t)cell_off[nc];
+    if (cells == 0 || periods < kTableLatency) return ATB_OK;
+    int occ[2] = {0, 0};
+    for (int w = 0; w < ga.vs; ++w) {
+        const GatherFn fn = gather_fn(p->prm.geometry, w == 0);
+        p->gather_smem[w] = kGatherWarps * ((int)gather_ring_bytes(ga.ring) + gather_state_bytes(w + 1));
+        ATB_CUDA(p->h, cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                            p->gather_smem[w]));
+        ATB_CUDA(p->h, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ[w], fn, kGatherBlock,
+                                                                     p->gather_smem[w]));
+        if (occ[w] < 1) return ATB_OK;
+    }
+    long long *d_cells = nullptr, *d_bits = nullptr, *d_flags = nullptr;
+    std::vector<long long> bit_off(nc + 1, 0), flag_off(nc + 1, 0);
+    for (int c = 0; c < nc; ++c) {
+        const bool has = p->prm.geometry == ATB_GEOM_BINNED && cell_off[c + 1] > cell_off[c];
+        int bl = 0;
+        while ((pt_off[c + 1] - pt_off[c]) >> bl) ++bl;
+        bit_off[c + 1] = bit_off[c] + (has ? offset_words(bl) : 0);
+        flag_off[c + 1] = flag_off[c] + per_cnt[c];
+    }
+    PlanArrays arr;
+    arr.upload(&d_cells, cell_off);
+    arr.upload(&d_bits, bit_off);
+    arr.upload(&d_flags, flag_off);
+    arr.scratch(&ga.tab, cells * 16 * ga.vs);
+    arr.scratch(&ga.idx, cells);
+    arr.scratch(&ga.bits, (size_t)bit_off[nc]);
+    arr.scratch(&p->tstats, (size_t)nc);
+    unsigned char* flags = nullptr;
+    arr.scratch(&flags, (size_t)flag_off[nc]);
+    if (arr.commit(p)) {
+        cudaGetLastError();
+        p->h->err.clear();
+        return ATB_OK;
+    }
+    p->qa.scatter = flags;
+    ga.bit_off = d_bits;
+    p->qa.flag_off = d_flags;
+    p->qa.tstats = p->tstats;
+    ga.cell_off = d_cells;
+    ga.counter = p->control->gathers;
+    ga.n_gather = p->control->n_gather;
+    ga.n_scatter = &p->control->n_scatter;
+    for (int w = 0; w < ga.vs; ++w)
+        p->gather_grid[w] =
+            (int)std::max(1LL, std::min((long long)p->h->n_sm * occ[w], 4 * p->n_tiles));
+    p->ga = ga;
+    p->qa.n_scatter = ga.n_scatter;
     return ATB_OK;
 }
 
@@ -2493,19 +2680,30 @@ int plan_create(atb_handle* h, const atb_params* prm, const atb_batch* b, const 
     double* d_sdt;
     int *d_sqw, *d_sqy;
     CurveStat* d_stats;
-    if ((rc = plan_upload(p, &d_pt, pt_off)) || (rc = plan_upload(p, &d_toff, t_off)) ||
-        (rc = plan_upload(p, &d_pbeg, per_beg)) || (rc = plan_upload(p, &d_pcnt, per_cnt)) ||
-        (rc = plan_upload(p, &d_dbeg, dur_beg)) || (rc = plan_upload(p, &d_obeg, out_beg)) ||
-        (rc = plan_upload(p, &d_soff, stage_off)) || (rc = plan_upload(p, &d_tiles, tile_off)) ||
-        (rc = plan_upload(p, &d_dcnt, dur_cnt)) || (rc = plan_upload(p, &d_order, order)) ||
-        (rc = plan_alloc(p, &d_dbins, (size_t)nc * kMaxDur)) ||
-        (rc = plan_alloc(p, &d_sdt, (size_t)staged)) || (rc = plan_alloc(p, &d_sqw, (size_t)staged)) ||
-        (rc = plan_alloc(p, &d_sqy, (size_t)staged)) || (rc = plan_alloc(p, &d_stats, (size_t)nc)) ||
-        (rc = plan_alloc(p, &p->status, 1)) || (rc = plan_alloc(p, &p->counter, 1))) {
+    PlanArrays arr;
+    arr.upload(&d_pt, pt_off);
+    arr.upload(&d_toff, t_off);
+    arr.upload(&d_pbeg, per_beg);
+    arr.upload(&d_pcnt, per_cnt);
+    arr.upload(&d_dbeg, dur_beg);
+    arr.upload(&d_obeg, out_beg);
+    arr.upload(&d_soff, stage_off);
+    arr.upload(&d_tiles, tile_off);
+    arr.upload(&d_dcnt, dur_cnt);
+    arr.upload(&d_order, order);
+    arr.scratch(&d_dbins, (size_t)nc * kMaxDur);
+    arr.scratch(&d_sdt, (size_t)staged);
+    arr.scratch(&d_sqw, (size_t)staged);
+    arr.scratch(&d_sqy, (size_t)staged);
+    arr.scratch(&d_stats, (size_t)nc);
+    arr.scratch(&p->control, 1);
+    if ((rc = arr.commit(p))) {
         plan_free(p);
         delete p;
         return rc;
     }
+
+    p->status = &p->control->status;
 
     StageArgs& sa = p->sa;
     sa.pt_off = d_pt;
@@ -2540,8 +2738,7 @@ int plan_create(atb_handle* h, const atb_params* prm, const atb_batch* b, const 
     int nb_max = prm->n_bins;
     if (prm->geometry == ATB_GEOM_BINNED) {
         // largest bin count over the batch sizes the global-histogram fallback
-        int* d_nb = nullptr;
-        if ((rc = plan_alloc(p, &d_nb, 1))) { plan_free(p); delete p; return rc; }
+        int* d_nb = &p->control->nb_max;
         cudaMemsetAsync(d_nb, 0, sizeof(int), stream);
         nbins_max_kernel<<<nc, 256, 0, stream>>>(nc, d_pbeg, d_pcnt, d_dbeg, d_dcnt, b->periods,
                                                  b->durations, prm->oversample, prm->max_bins,
@@ -2628,9 +2825,14 @@ int plan_create(atb_handle* h, const atb_params* prm, const atb_batch* b, const 
     qa.window = o->window;
     qa.ghist = d_ghist;
     qa.ghist_stride = gstride;
-    qa.tile_counter = p->counter;
+    qa.tile_counter = &p->control->tiles;
     qa.status = p->status;
     p->best = o->best_period;
+    if ((rc = plan_gather(p, pt_off, per_cnt, b->w != nullptr))) {
+        plan_free(p);
+        delete p;
+        return rc;
+    }
     // every set-up copy has completed (or, for asynchronous plans, is ordered
     // before the plan's kernels on its stream)
     if (!async) ATB_CUDA(h, cudaDeviceSynchronize());
@@ -2643,14 +2845,10 @@ int atb_plan_execute(atb_plan* p, void* stream) {
     if (!p) return ATB_EINVAL;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     atb_handle* h = p->h;
-    ATB_CUDA(h, cudaMemsetAsync(p->counter, 0, sizeof(unsigned long long), s));
-    ATB_CUDA(h, cudaMemsetAsync(p->status, 0, sizeof(int), s));
+    ATB_CUDA(h, cudaMemsetAsync(p->control, 0, sizeof(atb_plan::Control), s));
     int rc = launch_stage(p, s);
     if (rc) return rc;
-    if (p->n_tiles > 0) {
-        search_fn(p->prm.geometry, p->nt)<<<p->grid, p->nt, p->smem_bytes, s>>>(p->qa);
-        ATB_CUDA(h, cudaGetLastError());
-    }
+    if (p->n_tiles > 0 && (rc = launch_search(p, s))) return rc;
     if (p->best) {
         const int threads = 256;
         const int blocks = (p->n_curves * 32 + threads - 1) / threads;
@@ -2663,7 +2861,7 @@ int atb_plan_execute(atb_plan* p, void* stream) {
 
 int atb_plan_kernel_count(const atb_plan* p) {
     if (!p) return 0;
-    return 1 + (p->n_tiles > 0 ? 1 : 0) + (p->best ? 1 : 0);
+    return 1 + (p->n_tiles > 0 ? (p->ga.tab ? 2 + p->ga.vs : 1) : 0) + (p->best ? 1 : 0);
 }
 
 int64_t atb_plan_scratch_bytes(const atb_plan* p) { return p ? p->scratch_bytes : 0; }
@@ -2864,16 +3062,11 @@ int atb_plan_profile(atb_plan* p, void* stream, float* ms_stage, float* ms_searc
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     cudaEvent_t ev[4];
     for (auto& e : ev) ATB_CUDA(h, cudaEventCreate(&e));
-    ATB_CUDA(h, cudaMemsetAsync(p->counter, 0, sizeof(unsigned long long), s));
-    ATB_CUDA(h, cudaMemsetAsync(p->status, 0, sizeof(int), s));
+    ATB_CUDA(h, cudaMemsetAsync(p->control, 0, sizeof(atb_plan::Control), s));
     ATB_CUDA(h, cudaEventRecord(ev[0], s));
     int rc = launch_stage(p, s);
     ATB_CUDA(h, cudaEventRecord(ev[1], s));
-    if (!rc && p->n_tiles > 0) {
-        search_fn(p->prm.geometry, p->nt)<<<p->grid, p->nt, p->smem_bytes, s>>>(p->qa);
-        cudaError_t e = cudaGetLastError();
-        if (e != cudaSuccess) rc = fail(h, ATB_ECUDA, "search launch: %s", cudaGetErrorString(e));
-    }
+    if (!rc && p->n_tiles > 0) rc = launch_search(p, s);
     ATB_CUDA(h, cudaEventRecord(ev[2], s));
     if (!rc && p->best) {
         const int blocks = (p->n_curves * 32 + 255) / 256;

@@ -130,8 +130,13 @@ def check_request(t: np.ndarray, y: np.ndarray, dy, periods: np.ndarray,
 def request_bytes(n_points: int, n_periods: int, n_durations: int) -> int:
     """Device bytes a request holds while its batch runs: inputs (t f64, y, w
     f32), staged points (16 B), the grids and the per-period outputs (28 B),
-    rounded up for the plan's descriptors."""
-    return int(n_points * (16 + 16) + n_periods * (8 + 28) + n_durations * 8 + 4096)
+    rounded up for the plan's descriptors; curves of 4096 to 2^18 - 1 points also
+    the look-up table (two cells of 36 B and 16 B of offset bits per point, 2176
+    cells more per curve, a flag per period)."""
+    table = 0
+    if 4096 <= n_points < 1 << 18 and n_periods >= 32:
+        table = n_points * (2 * 36 + 16) + 2176 * 36 + n_periods
+    return int(n_points * (16 + 16) + n_periods * (8 + 28) + n_durations * 8 + 4096 + table)
 
 
 class BLSServer:
