@@ -19,6 +19,8 @@
 //                  (exact int64 -> exact FP64), evaluate every (start,
 //                  duration) window in FP32 with an exact rational
 //                  comparison, and re-evaluate the winner in FP64.
+//   table, gather  dense curves: the same search by table look-ups instead of
+//                  histograms (bls_gather.cuh), where that is cheaper.
 //   best kernel    per-curve argmax over the period grid.
 //
 // Reference semantics followed (paths within ubunbun18/Astro_Transit_GPU):
@@ -82,7 +84,13 @@ constexpr int kMaxDur = 32;            // durations per curve
 // unclamped one) and start + length never overflows an int.
 constexpr int kLenCap = 1 << 28;
 constexpr int kStageAlign = 32;        // staged curves start at multiples of 32 points
-constexpr int kStageBlock = 256;
+// Threads of a stage CTA (one CTA per curve): kStageBlock for up to kStageWide
+// curves, so that long curves of a small batch are staged in parallel (200 000 points
+// 1.11 -> 0.44 ms, one curve of 15 000 52 -> 41 us); more curves fill the GPU with
+// kStageBlockB each (2000 of 15 000 points: 0.57 against 0.60 ms).
+constexpr int kStageBlock = 1024;
+constexpr int kStageBlockB = 256;
+constexpr int kStageWide = 592;
 constexpr double kDefaultMergeRun = 8.0;   // atb_params.merge_run = 0
 // atb_params.cta_threads = 0 with fixed bins: four 256-thread CTAs per SM
 // (measured faster than two 512-thread ones for fixed bins; slower for the
@@ -356,7 +364,7 @@ __device__ __forceinline__ long long warp_sum(long long v) {
     return v;
 }
 
-// block reductions for the stage kernel (kStageBlock threads)
+// block reductions for the stage kernel (at most kStageBlock threads)
 __device__ double block_max_d(double v, double* sh) {
     v = warp_max(v);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -364,7 +372,7 @@ __device__ double block_max_d(double v, double* sh) {
     if (lane == 0) sh[warp] = v;
     __syncthreads();
     double r = sh[0];
-    for (int i = 1; i < kStageBlock / 32; ++i) r = max(r, sh[i]);
+    for (int i = 1; i < (int)blockDim.x / 32; ++i) r = max(r, sh[i]);
     return r;
 }
 
@@ -375,7 +383,7 @@ __device__ long long block_sum_ll(long long v, long long* sh) {
     if (lane == 0) sh[warp] = v;
     __syncthreads();
     long long r = 0;
-    for (int i = 0; i < kStageBlock / 32; ++i) r += sh[i];
+    for (int i = 0; i < (int)blockDim.x / 32; ++i) r += sh[i];
     return r;
 }
 
@@ -394,13 +402,13 @@ __device__ int occupancy_bits(const StageArgs& a, int c, const double* t, long l
                               long long* shl) {
     // time order
     int unsorted = 0;
-    for (long long i = threadIdx.x; i + 1 < n; i += kStageBlock) unsorted |= t[i] > t[i + 1];
+    for (long long i = threadIdx.x; i + 1 < n; i += (int)blockDim.x) unsorted |= t[i] > t[i + 1];
     if (__syncthreads_or(unsorted)) return 64;
     // grid extremes
     const double* per = a.periods + a.per_beg[c];
     const long long np = a.per_cnt[c];
     double pmax = 0.0, pinv = 0.0;
-    for (long long i = threadIdx.x; i < np; i += kStageBlock) {
+    for (long long i = threadIdx.x; i < np; i += (int)blockDim.x) {
         const double P = per[i];
         if (P > 0.0 && P < 1.0e300) {
             pmax = max(pmax, P);
@@ -428,7 +436,7 @@ __device__ int occupancy_bits(const StageArgs& a, int c, const double* t, long l
     if (!(width > 0.0) || !isfinite(width)) return 64;
     width = width * (1.0 + 1e-6) + 1e-12;
     // K: each thread scans a contiguous range of window starts with a second pointer
-    const long long per_thr = (n + kStageBlock - 1) / kStageBlock;
+    const long long per_thr = (n + (int)blockDim.x - 1) / (int)blockDim.x;
     const long long i0 = min(n, (long long)threadIdx.x * per_thr);
     const long long i1 = min(n, i0 + per_thr);
     long long kmax = 0;
@@ -462,7 +470,7 @@ __device__ bool checked_tight_ok(const StageArgs& a, int c, long long n, double*
     const double* per = a.periods + a.per_beg[c];
     const long long np = a.per_cnt[c];
     double pmax = 0.0, pinv = 0.0;
-    for (long long i = threadIdx.x; i < np; i += kStageBlock) {
+    for (long long i = threadIdx.x; i < np; i += (int)blockDim.x) {
         const double P = per[i];
         if (P > 0.0 && P < 1.0e300) {
             pmax = max(pmax, P);
@@ -505,7 +513,7 @@ __global__ void __launch_bounds__(kStageBlock) stage_kernel(const StageArgs a) {
     // pass 1: magnitudes and validity
     double wmax = 0.0, amax = 0.0, tmax = 0.0;
     int bad = 0;
-    for (long long i = threadIdx.x; i < n; i += kStageBlock) {
+    for (long long i = threadIdx.x; i < n; i += (int)blockDim.x) {
         const double wi = w ? (double)w[i] : 1.0;
         const double yi = (double)y[i];
         if (!(wi > 0.0) || !isfinite(wi) || !isfinite(yi) || !isfinite(t[i])) bad = 1;
@@ -524,7 +532,7 @@ __global__ void __launch_bounds__(kStageBlock) stage_kernel(const StageArgs a) {
     // range of the quantised weights decides the histogram layout
     long long sqw = 0, sqa = 0;
     int qw_min = 0x7fffffff, qw_max = -1;
-    for (long long i = threadIdx.x; i < n; i += kStageBlock) {
+    for (long long i = threadIdx.x; i < n; i += (int)blockDim.x) {
         const double wi = w ? (double)w[i] : 1.0;
         const double yi = (double)y[i];
         const long long qa = __double2ll_rn(ldexp(wi, s_w));
@@ -555,7 +563,7 @@ __global__ void __launch_bounds__(kStageBlock) stage_kernel(const StageArgs a) {
 
     // pass 3: magnitude of w*(y - c)
     double vmax = 0.0;
-    for (long long i = threadIdx.x; i < n; i += kStageBlock) {
+    for (long long i = threadIdx.x; i < n; i += (int)blockDim.x) {
         const double wi = w ? (double)w[i] : 1.0;
         vmax = max(vmax, fabs(wi * ((double)y[i] - shift)));
     }
@@ -587,7 +595,7 @@ __global__ void __launch_bounds__(kStageBlock) stage_kernel(const StageArgs a) {
     const bool ilv = n > 1 && width > 0.0 && tmax >= width * (double)(n - 1);
     const long long n_full = ilv ? n_pad / kChunk * kChunk : 0;
     long long qw_tot = 0, qy_tot = 0, qy_abs = 0;
-    for (long long i = threadIdx.x; i < n_pad; i += kStageBlock) {
+    for (long long i = threadIdx.x; i < n_pad; i += (int)blockDim.x) {
         double d = 0.0;
         int qa = 0, qb = 0;
         if (i < n) {
@@ -2279,9 +2287,11 @@ int plan_alloc(atb_plan* p, T** out, size_t count) {
     return ATB_OK;
 }
 
-// A plan's device arrays in one allocation, its host index arrays in one copy: a
-// plan of one curve is made for every call of the per-call API, where each
-// separate allocation and copy costs several microseconds of host time.
+// A plan's device arrays, its host index arrays in one copy.  A stream-ordered plan
+// -- one is made for every call of the per-call API, where each allocation and
+// copy costs several microseconds of host time -- takes everything in one
+// allocation.  Other plans take the scratch arrays one by one: cudaMalloc serves blocks
+// below a megabyte or so from mapped memory, and would map and unmap a larger one.
 struct PlanArrays {
     std::vector<std::pair<void**, size_t>> slots;  // pointer to set, byte offset
     std::vector<char> host;                        // the uploads (they come first)
@@ -2304,9 +2314,17 @@ struct PlanArrays {
     }
     int commit(atb_plan* p) {
         char* base = nullptr;
-        int rc = plan_alloc(p, &base, bytes);
+        int rc = plan_alloc(p, &base, p->async ? bytes : host.size());
         if (rc) return rc;
-        for (auto& s : slots) *s.first = base + s.second;
+        for (size_t i = 0; i < slots.size(); ++i) {
+            const size_t at = slots[i].second;
+            char* q = base + at;
+            if (!p->async && at >= host.size()) {
+                const size_t end = i + 1 < slots.size() ? slots[i + 1].second : bytes;
+                if ((rc = plan_alloc(p, &q, end - at))) return rc;
+            }
+            *slots[i].first = q;
+        }
         // from pageable memory: returns once the data are staged, so `host` may go
         if (!host.empty())
             ATB_CUDA(p->h, p->async ? cudaMemcpyAsync(base, host.data(), host.size(),
@@ -2369,10 +2387,11 @@ bool plan_shape(const atb_params* prm, int* nt, int* minb) {
 }
 
 int launch_stage(atb_plan* p, cudaStream_t s) {
+    const int nt = p->n_curves <= kStageWide ? kStageBlock : kStageBlockB;
     if (p->y_is_f64)
-        stage_kernel<double><<<p->n_curves, kStageBlock, 0, s>>>(p->sa);
+        stage_kernel<double><<<p->n_curves, nt, 0, s>>>(p->sa);
     else
-        stage_kernel<float><<<p->n_curves, kStageBlock, 0, s>>>(p->sa);
+        stage_kernel<float><<<p->n_curves, nt, 0, s>>>(p->sa);
     ATB_CUDA(p->h, cudaGetLastError());
     return ATB_OK;
 }
@@ -2461,7 +2480,16 @@ int plan_gather(atb_plan* p, const std::vector<long long>& pt_off,
     arr.scratch(&p->tstats, (size_t)nc);
     unsigned char* flags = nullptr;
     arr.scratch(&flags, (size_t)flag_off[nc]);
-    if (arr.commit(p)) {
+    const size_t held = p->allocs.size();
+    const long long held_bytes = p->scratch_bytes;
+    if (arr.commit(p)) {  // give back what it did get
+        while (p->allocs.size() > held) {
+            if (p->async) cudaFreeAsync(p->allocs.back(), p->stream);
+            else cudaFree(p->allocs.back());
+            p->allocs.pop_back();
+        }
+        p->scratch_bytes = held_bytes;
+        p->tstats = nullptr;
         cudaGetLastError();
         p->h->err.clear();
         return ATB_OK;

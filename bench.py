@@ -653,13 +653,12 @@ def main(argv=None):
             "bound": "smem",
             "kernel": "search_kernel<FIXED>" if args.method == "fast" else "search_kernel<BINNED>",
             "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
-            "traffic": measured_traffic(
-                args.workload, args.method, nc,
-                search_algorithmic_bytes(lens, [len(curve_periods(periods, c))
-                                                for c in range(nc)])),
-            "traffic_source": "ncu capture of a smaller launch of this workload under profiles/, "
-                              "scaled to this launch (null: no capture of this workload)",
-            "units": "4 B per 32-bit shared-memory reduction the fold issues: 2, 3 or 4 per "
+            "traffic": None,
+            "traffic_source": "no capture of this launch: the committed ones are of the scatter "
+                              "kernel alone",
+            "units": "4 B per 32-bit shared-memory reduction of the scattered form of the search, "
+                     "whether the engine scattered or gathered the curve (gathered curves issue "
+                     "table look-ups instead): 2, 3 or 4 per "
                      "(point, period) update by the curve's histogram layout (tight, count, "
                      f"split; a checked tight period that is folded again counts 2); "
                      f"{u_fold:.3e} updates and {red_bytes / 4:.3e} reductions per launch",
