@@ -413,7 +413,9 @@ __global__ void __launch_bounds__(kTableBlock) table_kernel(const SearchArgs a, 
         n_g = tb_sum(n_g, sh);
         saved = tb_sum(saved, sh);
     }
-    on = saved * min(a.n_curves, 600) >= kTableLatency * n;
+    // (what was refused above stays refused: a curve without points has no cells to write
+    // to, and its zero savings would meet its zero price)
+    on = on && saved * min(a.n_curves, 600) >= kTableLatency * n;
     if (on) {
         const int bl = bitlen64(n);
         // the padding copy can repeat every point once: counts below 2^(bl + 1), flux

@@ -1,0 +1,74 @@
+"""GPU tests of the prefix-gather search on batches of unlike curves.
+
+The search tables of a batch lie one after another in shared arrays, so a curve
+that is not gathered must leave its neighbours' tables alone, and its own periods
+must go to the scatter kernel.  Every comparison is exact: the search sums are
+integers, whichever kernel takes a period.
+"""
+import numpy as np
+import pytest
+
+import recipes as R
+from oracle import oracle as O
+
+pytestmark = pytest.mark.gpu
+
+FIELDS = ("power", "depth", "depth_err", "t0", "duration", "window")
+DURS = np.array([0.04, 0.06, 0.08, 0.12, 0.16, 0.20])
+CHECKED = np.array([0.9, 1.999, 3.71, 5.0, 9.13, 12.4, 13.7, 27.0])
+N_PER = 1600
+
+
+@pytest.fixture(scope="module")
+def engine():
+    from astro_transit_gpu_b200.engine import BLSEngine
+    return BLSEngine.get()
+
+
+def config(kind, n_bins=200):
+    from astro_transit_gpu_b200.engine import SearchConfig
+    if kind == "fixed":
+        return SearchConfig("fast", n_bins=n_bins)
+    return SearchConfig("parity", objective="likelihood")
+
+
+def grid(kind):
+    """The checked periods and fillers whose look-ups are few against their points."""
+    lo, hi = (6.0, 13.0) if kind == "fixed" else (0.9, 2.2)
+    return np.concatenate([CHECKED, np.geomspace(lo, hi, N_PER - len(CHECKED))])
+
+
+def dense_curve(seed, n=14001):
+    rng = np.random.default_rng(seed)
+    g = R.cadence_grid()
+    t = g[:n] + 0.0055 * np.sin(2 * np.pi * g[:n] / 365.25 + seed)
+    y = 1.0 + rng.normal(0.0, 1e-3, n)
+    return t, R.inject_box(t, y, 3.71, t[0] + 1.2, 0.10, 1.5e-3).astype(np.float32)
+
+
+def oracle_outputs(kind, t, y, w):
+    if kind == "fixed":
+        return O.eng_fixed(t, y, w, CHECKED, DURS, n_bins=200)
+    return O.eng_binned(t, y, w, CHECKED, DURS, objective="likelihood")
+
+
+@pytest.mark.parametrize("weighted", [False, True])
+@pytest.mark.parametrize("kind", ["binned", "fixed"])
+def test_empty_curves_between_dense_ones(engine, kind, weighted):
+    """A curve without points gives zeros and leaves its neighbours' results alone."""
+    from astro_transit_gpu_b200.engine import CurveBatch, split_outputs
+    a, b = dense_curve(1), dense_curve(2, 14337)
+    none = (np.zeros(0), np.zeros(0, np.float32))
+    curves = [none] + [a, b] * 12 + [none, none] + [b, a] * 12 + [none]
+    weight = lambda c: np.full(len(c[0]), 1.0e6, np.float32)  # noqa: E731
+    batch = CurveBatch.from_arrays([c[0] for c in curves], [c[1] for c in curves],
+                                   periods=grid(kind), durations=DURS,
+                                   weights=[weight(c) for c in curves] if weighted else None)
+    outs = split_outputs(batch, engine.search(batch, config(kind)))
+    want = {id(c): oracle_outputs(kind, *c, weight(c) if weighted else None) for c in (a, b)}
+    for c, o in zip(curves, outs):
+        for f in FIELDS:
+            if c is none:
+                assert np.all(o[f] == (-1 if f == "window" else 0)), f
+            else:
+                assert np.array_equal(o[f][:len(CHECKED)], want[id(c)][f]), f
