@@ -2435,7 +2435,7 @@ int plan_gather(atb_plan* p, const std::vector<long long>& pt_off,
     if (p->prm.geometry == ATB_GEOM_FIXED) {
         // (entries up to two periods: windows that wrap)
         ga.ring = (2 * std::min(p->prm.n_bins, 1 << 20) + 2 + 31) / 32 * 32;
-        if (ga.ring > 1024) return ATB_OK;
+        if (ga.ring > kMaxRing) return ATB_OK;
     } else if (p->prm.oversample >= kHeadMax) {
         return ATB_OK;
     }
@@ -2454,9 +2454,12 @@ int plan_gather(atb_plan* p, const std::vector<long long>& pt_off,
     int occ[2] = {0, 0};
     for (int w = 0; w < ga.vs; ++w) {
         const GatherFn fn = gather_fn(p->prm.geometry, w == 0);
-        p->gather_smem[w] = kGatherWarps * ((int)gather_ring_bytes(ga.ring) + gather_state_bytes(w + 1));
+        p->gather_smem[w] = gather_smem_bytes(ga.ring, w + 1);
+        // the limit belongs to the kernel, not to the plan: the same for every
+        // plan, or a later plan with a shorter buffer would lower it below
+        // what an earlier one still launches with
         ATB_CUDA(p->h, cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                            p->gather_smem[w]));
+                                            gather_smem_bytes(kMaxRing, w + 1)));
         ATB_CUDA(p->h, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ[w], fn, kGatherBlock,
                                                                      p->gather_smem[w]));
         if (occ[w] < 1) return ATB_OK;

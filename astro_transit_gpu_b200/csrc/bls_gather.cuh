@@ -560,6 +560,7 @@ struct GatherPeriod {
     int period;        // index in the curve's grid
 };
 
+constexpr int kMaxRing = 1024;  // longest buffer of prefix entries (fixed bins)
 constexpr int kMaxPop = 4;    // periods of a tile a warp sets up together
 constexpr int kMaxCyc = 64;   // cycles whose table positions a warp holds
 constexpr int kMaxList = 64;  // windows within reach of the best, before the exact test
@@ -606,6 +607,11 @@ __host__ __device__ inline unsigned gather_ring_bytes(int ring) { return 8u * (r
 
 __host__ __device__ inline int gather_state_bytes(int vs) {
     return (int)(vs == 1 ? sizeof(WarpState<true>) : sizeof(WarpState<false>)) / 16 * 16 + 16;
+}
+
+// dynamic shared memory of a CTA of the gather kernel
+inline int gather_smem_bytes(int ring, int vs) {
+    return kGatherWarps * ((int)gather_ring_bytes(ring) + gather_state_bytes(vs));
 }
 
 // Look-up of the boundary at offset f of an entry's cell: V before the cell,

@@ -72,3 +72,23 @@ def test_empty_curves_between_dense_ones(engine, kind, weighted):
                 assert np.all(o[f] == (-1 if f == "window" else 0)), f
             else:
                 assert np.array_equal(o[f][:len(CHECKED)], want[id(c)][f]), f
+
+
+def test_plans_of_other_bin_counts_leave_a_plan_usable(engine):
+    """The gather kernel's shared memory grows with the bin count; plans of fewer
+    and of more bins, made later, must not change what an earlier plan may use."""
+    from astro_transit_gpu_b200.engine import CurveBatch, split_outputs
+    t, y = dense_curve(3)
+    batch = CurveBatch.from_arrays([t] * 8, [y] * 8, periods=grid("fixed"), durations=DURS)
+    plans = [engine.plan(batch, config("fixed", n)) for n in (500, 100, 300)]
+    want = [O.eng_fixed(t, y, None, CHECKED, DURS, n_bins=n) for n in (500, 100, 300)]
+    try:
+        for i in (0, 2, 1, 0):
+            plans[i].execute()
+            plans[i].check()
+            for o in split_outputs(batch, plans[i].outputs):
+                for f in FIELDS:
+                    assert np.array_equal(o[f][:len(CHECKED)], want[i][f]), (i, f)
+    finally:
+        for p in plans:
+            p.close()
