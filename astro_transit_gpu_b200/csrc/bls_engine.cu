@@ -2232,8 +2232,9 @@ struct atb_plan {
     struct Control {
         unsigned long long tiles;    // search kernel's work counter
         unsigned long long gathers[2];  // gather kernels' (packed, weighted)
+        unsigned long long n_gather[2];  // periods gathered (packed, weighted curves)
+        int n_scatter;               // some period is scattered
         int status;
-        int n_gather[2], n_scatter;     // some period is gathered / scattered
         int nb_max;                  // set-up: the largest bin count
     };
     Control* control = nullptr;

@@ -102,7 +102,7 @@ struct GatherArgs {
     const long long* bit_off;  // per curve: first word of `bits`
     const long long* cell_off; // per curve: first cell; cell_off[n_curves] = all
     unsigned long long* counter;  // work counters of the packed and the weighted kernel
-    int* n_gather;             // periods that are gathered, by kernel
+    unsigned long long* n_gather;  // periods that are gathered, by kernel
     int* n_scatter;            // some period is scattered
     int vs;                    // 2 when weights are given, else 1
     int ring;                  // prefix entries a warp holds
@@ -536,7 +536,7 @@ __global__ void __launch_bounds__(kTableBlock) table_kernel(const SearchArgs a, 
     if (tid == 0) {
         sg.g_on = on ? 1 : 0;
         stats[c] = sg;
-        if (on) atomicAdd(ga.n_gather + (st.cnt_win ? 0 : 1), (int)n_g);
+        if (on) atomicAdd(ga.n_gather + (st.cnt_win ? 0 : 1), (unsigned long long)n_g);
         if (!on || n_g < np) atomicOr(ga.n_scatter, 1);
     }
 }
@@ -1504,7 +1504,7 @@ __global__ void __launch_bounds__(kGatherBlock, kGatherMinBlocks)
         __syncthreads();
         if (threadIdx.x == 0) {
             int chunk = kGatherWarps * kMaxPop;
-            while (chunk > kGatherWarps && ga.n_gather[PK ? 0 : 1] / chunk < 16 * (int)gridDim.x)
+            while (chunk > kGatherWarps && ga.n_gather[PK ? 0 : 1] / chunk < 16 * gridDim.x)
                 chunk /= 2;
             const unsigned subs = (unsigned)((a.tile_p + chunk - 1) / chunk);
             const unsigned long long units = (unsigned long long)a.n_tiles * subs;

@@ -92,3 +92,36 @@ def test_plans_of_other_bin_counts_leave_a_plan_usable(engine):
     finally:
         for p in plans:
             p.close()
+
+
+def test_more_gathered_periods_than_32_bits_count(engine):
+    """2^16 targets screened over 2^16 periods: 2^32 gathered periods.  The periods
+    exceed the time span and the bins are two, so each takes 128 look-ups."""
+    import torch
+    from astro_transit_gpu_b200.engine import CurveBatch
+    nc, n, n_per = 1 << 16, 4096, 1 << 16
+    dev = engine.device
+    t = np.arange(n) * 0.01
+    periods = np.geomspace(1.1, 3.0, n_per) * t[-1]
+    dur = np.array([0.2 * t[-1]])
+    gen = torch.Generator(dev).manual_seed(5)
+    y = torch.randn(nc * n, generator=gen, device=dev, dtype=torch.float32)
+    batch = CurveBatch(
+        t=torch.from_numpy(t).to(dev), y=y, w=None, periods=torch.from_numpy(periods).to(dev),
+        durations=torch.from_numpy(dur).to(dev), point_offset=np.arange(nc + 1, dtype=np.int64) * n,
+        period_begin=np.zeros(nc, np.int64), period_count=np.full(nc, n_per, np.int64),
+        dur_begin=np.zeros(nc, np.int64), dur_count=np.ones(nc, np.int32),
+        out_begin=np.zeros(nc, np.int64), time_offset=np.zeros(nc, np.int64))
+    key = torch.zeros(nc, dtype=torch.int64, device=dev)
+    best = torch.empty(nc, dtype=torch.int32, device=dev)
+    plan = engine.plan(batch, config("fixed", 2), {"best_key": key, "best_period": best})
+    try:
+        plan.execute()
+        plan.check()
+    finally:
+        plan.close()
+    got = best.cpu().numpy()
+    assert got.min() >= 0
+    for c in (0, 1, nc // 2, nc - 1):
+        o = O.eng_fixed(t, y[c * n:(c + 1) * n].cpu().numpy(), None, periods, dur, n_bins=2)
+        assert got[c] == np.argmax(o["power"]), c
