@@ -34,6 +34,7 @@ EXPORTS = (
     "atb_run_vbls_exact_parity", "atb_debug_fold", "atb_plan_profile",
     "atb_bench_smem_red_u64", "atb_bench_smem_red_u32", "atb_bench_dfma", "atb_search_curve_static",
     "atb_plan_curve_layout", "atb_plan_create_async", "atb_plan_top_k",
+    "atb_plan_create_limited", "atb_plan_gathered",
 )
 
 # limit of atb_search_curve_static (ATB_STATIC_MAX_POINTS in the header)
@@ -98,6 +99,10 @@ def load(build_if_missing: bool = True):
                                       ctypes.POINTER(Outputs), ctypes.POINTER(_vp)]
         L.atb_plan_create_async.argtypes = [_vp, ctypes.POINTER(Params), ctypes.POINTER(Batch),
                                             ctypes.POINTER(Outputs), _vp, ctypes.POINTER(_vp)]
+        L.atb_plan_create_limited.argtypes = [_vp, ctypes.POINTER(Params), ctypes.POINTER(Batch),
+                                              ctypes.POINTER(Outputs), _vp, _i64,
+                                              ctypes.POINTER(_vp)]
+        L.atb_plan_gathered.argtypes = [_vp, _i64p, _i64p, _i64p]
         L.atb_plan_execute.argtypes = [_vp, _vp]
         L.atb_plan_top_k.argtypes = [_vp, _i32, _i32, _vp, _vp]
         L.atb_plan_check.argtypes = [_vp]
@@ -128,6 +133,7 @@ def load(build_if_missing: bool = True):
         for fn in ("atb_search_curve_static", "atb_plan_profile", "atb_bench_smem_red_u64",
                    "atb_bench_smem_red_u32", "atb_bench_dfma",
                    "atb_create", "atb_last_error", "atb_plan_create", "atb_plan_create_async",
+                   "atb_plan_create_limited", "atb_plan_gathered",
                    "atb_plan_execute", "atb_plan_top_k",
                    "atb_plan_check", "atb_plan_kernel_count", "atb_search", "atb_run_gpu_bls",
                    "atb_run_vbls_exact_parity", "atb_debug_fold"):

@@ -2233,6 +2233,7 @@ struct atb_plan {
         unsigned long long tiles;    // search kernel's work counter
         unsigned long long gathers[2];  // gather kernels' (packed, weighted)
         unsigned long long n_gather[2];  // periods gathered (packed, weighted curves)
+        unsigned long long n_back;   // of these, left to the scatter kernel after all
         int n_scatter;               // some period is scattered
         int status;
         int nb_max;                  // set-up: the largest bin count
@@ -2426,9 +2427,11 @@ int launch_search(atb_plan* p, cudaStream_t s) {
 }
 
 // Tables and launch shape of the gather kernel.  Without memory for the
-// tables the plan scatters every period.
+// tables, or where they would take more than `limit` bytes (negative: no limit), the
+// plan scatters every period.
 int plan_gather(atb_plan* p, const std::vector<long long>& pt_off,
-                const std::vector<long long>& per_cnt, bool weighted) {
+                const std::vector<long long>& per_cnt, bool weighted, long long limit) {
+    if (limit == 0) return ATB_OK;
     const int nc = p->n_curves;
     GatherArgs ga{};
     ga.vs = weighted ? 2 : 1;
@@ -2484,6 +2487,7 @@ int plan_gather(atb_plan* p, const std::vector<long long>& pt_off,
     arr.scratch(&p->tstats, (size_t)nc);
     unsigned char* flags = nullptr;
     arr.scratch(&flags, (size_t)flag_off[nc]);
+    if (limit > 0 && arr.bytes > (size_t)limit) return ATB_OK;
     const size_t held = p->allocs.size();
     const long long held_bytes = p->scratch_bytes;
     if (arr.commit(p)) {  // give back what it did get
@@ -2505,6 +2509,7 @@ int plan_gather(atb_plan* p, const std::vector<long long>& pt_off,
     ga.cell_off = d_cells;
     ga.counter = p->control->gathers;
     ga.n_gather = p->control->n_gather;
+    ga.n_back = &p->control->n_back;
     ga.n_scatter = &p->control->n_scatter;
     for (int w = 0; w < ga.vs; ++w)
         p->gather_grid[w] =
@@ -2593,22 +2598,28 @@ int atb_last_error(const atb_handle* h, char* buf, size_t len) {
 
 namespace {
 int plan_create(atb_handle* h, const atb_params* prm, const atb_batch* b, const atb_outputs* o,
-                cudaStream_t stream, bool async, atb_plan** out);
+                cudaStream_t stream, bool async, long long table_bytes, atb_plan** out);
 }  // namespace
 
 int atb_plan_create(atb_handle* h, const atb_params* prm, const atb_batch* b,
                     const atb_outputs* o, atb_plan** out) {
-    return plan_create(h, prm, b, o, nullptr, false, out);
+    return plan_create(h, prm, b, o, nullptr, false, -1, out);
 }
 
 int atb_plan_create_async(atb_handle* h, const atb_params* prm, const atb_batch* b,
                           const atb_outputs* o, void* stream, atb_plan** out) {
-    return plan_create(h, prm, b, o, static_cast<cudaStream_t>(stream), true, out);
+    return plan_create(h, prm, b, o, static_cast<cudaStream_t>(stream), true, -1, out);
+}
+
+int atb_plan_create_limited(atb_handle* h, const atb_params* prm, const atb_batch* b,
+                            const atb_outputs* o, void* stream, int64_t table_bytes,
+                            atb_plan** out) {
+    return plan_create(h, prm, b, o, static_cast<cudaStream_t>(stream), true, table_bytes, out);
 }
 
 namespace {
 int plan_create(atb_handle* h, const atb_params* prm, const atb_batch* b, const atb_outputs* o,
-                cudaStream_t stream, bool async, atb_plan** out) {
+                cudaStream_t stream, bool async, long long table_bytes, atb_plan** out) {
     if (!h) return ATB_EINVAL;
     if (!prm || !b || !o || !out) return fail(h, ATB_EINVAL, "null argument");
     *out = nullptr;
@@ -2860,7 +2871,7 @@ int plan_create(atb_handle* h, const atb_params* prm, const atb_batch* b, const 
     qa.tile_counter = &p->control->tiles;
     qa.status = p->status;
     p->best = o->best_period;
-    if ((rc = plan_gather(p, pt_off, per_cnt, b->w != nullptr))) {
+    if ((rc = plan_gather(p, pt_off, per_cnt, b->w != nullptr, table_bytes))) {
         plan_free(p);
         delete p;
         return rc;
@@ -2894,6 +2905,19 @@ int atb_plan_execute(atb_plan* p, void* stream) {
 int atb_plan_kernel_count(const atb_plan* p) {
     if (!p) return 0;
     return 1 + (p->n_tiles > 0 ? (p->ga.tab ? 2 + p->ga.vs : 1) : 0) + (p->best ? 1 : 0);
+}
+
+int atb_plan_gathered(atb_plan* p, int64_t* counting, int64_t* weighted, int64_t* given_back) {
+    if (!p || !counting || !weighted || !given_back) return ATB_EINVAL;
+    *counting = *weighted = *given_back = 0;
+    if (!p->ga.tab) return ATB_OK;
+    ATB_CUDA(p->h, cudaSetDevice(p->h->device));
+    atb_plan::Control ctl;
+    ATB_CUDA(p->h, plan_read(p, &ctl, p->control, sizeof ctl));
+    *counting = (int64_t)ctl.n_gather[0];
+    *weighted = (int64_t)ctl.n_gather[1];
+    *given_back = (int64_t)ctl.n_back;
+    return ATB_OK;
 }
 
 int64_t atb_plan_scratch_bytes(const atb_plan* p) { return p ? p->scratch_bytes : 0; }

@@ -103,6 +103,7 @@ struct GatherArgs {
     const long long* cell_off; // per curve: first cell; cell_off[n_curves] = all
     unsigned long long* counter;  // work counters of the packed and the weighted kernel
     unsigned long long* n_gather;  // periods that are gathered, by kernel
+    unsigned long long* n_back;    // of these, given back to the scatter kernel
     int* n_scatter;            // some period is scattered
     int vs;                    // 2 when weights are given, else 1
     int ring;                  // prefix entries a warp holds
@@ -1480,6 +1481,7 @@ __device__ __forceinline__ void gather_periods(const SearchArgs& a, const Gather
         if (!(done >> lane & 1u)) {  // left to the scatter kernel
             a.scatter[a.flag_off[c] + ws.per[lane].period] = 1;
             atomicOr(ga.n_scatter, 1);
+            atomicAdd(ga.n_back, 1ULL);
         }
     }
     __syncwarp();

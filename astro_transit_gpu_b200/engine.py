@@ -203,9 +203,13 @@ class SearchPlan:
     """A batch bound to output tensors; ``execute`` enqueues the search."""
 
     def __init__(self, engine: "BLSEngine", batch: CurveBatch, config: SearchConfig,
-                 outputs: Dict[str, torch.Tensor], stream: Optional[torch.cuda.Stream] = None):
+                 outputs: Dict[str, torch.Tensor], stream: Optional[torch.cuda.Stream] = None,
+                 table_bytes: int = -1):
         """With `stream`, the plan is set up and released in that stream's
-        order (atb_plan_create_async) and must be executed on it."""
+        order (atb_plan_create_async) and must be executed on it; `table_bytes`
+        then limits its look-up tables (atb_plan_create_limited)."""
+        if stream is None and table_bytes >= 0:
+            raise ValueError("table_bytes needs a stream")
         self.engine = engine
         self.stream = stream
         self.batch = batch
@@ -243,10 +247,10 @@ class SearchPlan:
                 rc = lib.atb_plan_create(engine.handle.ptr, ctypes.byref(self._params),
                                          ctypes.byref(b), ctypes.byref(o), ctypes.byref(ptr))
             else:
-                rc = lib.atb_plan_create_async(engine.handle.ptr, ctypes.byref(self._params),
-                                               ctypes.byref(b), ctypes.byref(o),
-                                               ctypes.c_void_p(stream.cuda_stream),
-                                               ctypes.byref(ptr))
+                rc = lib.atb_plan_create_limited(engine.handle.ptr, ctypes.byref(self._params),
+                                                 ctypes.byref(b), ctypes.byref(o),
+                                                 ctypes.c_void_p(stream.cuda_stream),
+                                                 int(table_bytes), ctypes.byref(ptr))
         N.raise_for(rc, engine.handle.ptr, "plan creation")
         self.ptr = ptr
 
@@ -300,6 +304,15 @@ class SearchPlan:
             bits.ctypes.data_as(ctypes.POINTER(ctypes.c_int32)))
         N.raise_for(rc, self.engine.handle.ptr, "curve layout")
         return lay, bits
+
+    def gathered(self) -> Dict[str, int]:
+        """After an execution: how many periods the look-up search took of curves
+        of equal ("counting") and unequal weights ("weighted"), and how many of
+        these it gave back to the histogram search ("given_back").  Synchronous."""
+        v = [ctypes.c_int64(0) for _ in range(3)]
+        rc = self._lib.atb_plan_gathered(self.ptr, *(ctypes.byref(x) for x in v))
+        N.raise_for(rc, self.engine.handle.ptr, "gathered periods")
+        return {"counting": v[0].value, "weighted": v[1].value, "given_back": v[2].value}
 
     def check(self) -> None:
         """Synchronise and raise ValueError if the last execution saw invalid data."""
@@ -457,10 +470,11 @@ class BLSEngine:
 
     def plan(self, batch: CurveBatch, config: SearchConfig,
              outputs: Optional[Dict[str, torch.Tensor]] = None,
-             stream: Optional[torch.cuda.Stream] = None) -> SearchPlan:
+             stream: Optional[torch.cuda.Stream] = None, table_bytes: int = -1) -> SearchPlan:
         if outputs is None:
             outputs = self.allocate_outputs(batch)
-        return SearchPlan(self, batch, self.tuned_config(batch, config), outputs, stream)
+        return SearchPlan(self, batch, self.tuned_config(batch, config), outputs, stream,
+                          table_bytes)
 
     def screen(self, batch: CurveBatch, config: SearchConfig,
                stream: Optional[torch.cuda.Stream] = None) -> Dict[str, torch.Tensor]:

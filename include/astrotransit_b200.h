@@ -148,6 +148,17 @@ int atb_plan_create(atb_handle* h, const atb_params* params, const atb_batch* ba
  */
 int atb_plan_create_async(atb_handle* h, const atb_params* params, const atb_batch* batch,
                           const atb_outputs* outputs, void* stream, atb_plan** out);
+/*
+ * The plan of atb_plan_create_async with a limit on its look-up tables (no
+ * reference counterpart; results do not depend on it).  Dense curves are
+ * searched by look-ups in per-curve tables, 40 to 88 bytes per point of
+ * scratch; a plan whose tables would take more than table_bytes makes none
+ * and searches every period with shared-memory histograms.  0 = no tables,
+ * negative = no limit.
+ */
+int atb_plan_create_limited(atb_handle* h, const atb_params* params, const atb_batch* batch,
+                            const atb_outputs* outputs, void* stream, int64_t table_bytes,
+                            atb_plan** out);
 int atb_plan_execute(atb_plan* p, void* stream);
 /* Synchronises `stream`-independent plan state: returns ATB_EDATA if the last
    execution met invalid input data, ATB_OK otherwise. */
@@ -186,6 +197,15 @@ int atb_plan_top_k(atb_plan* p, int32_t k, int32_t distance, int32_t* out_idx, v
 #define ATB_LAYOUT_TIGHT 2
 #define ATB_LAYOUT_TIGHT_CHECKED 3
 int atb_plan_curve_layout(atb_plan* p, int32_t* layout, int32_t* occupancy_bits);
+
+/*
+ * Diagnostics: after an atb_plan_execute has completed, how many of its periods
+ * (of all curves) the look-up search took, for curves of equal weights
+ * (`counting`) and of unequal ones (`weighted`), and how many of these it gave
+ * back to the histogram search (too many windows within rounding of the best:
+ * a flat light curve).  Synchronous.
+ */
+int atb_plan_gathered(atb_plan* p, int64_t* counting, int64_t* weighted, int64_t* given_back);
 
 /* One-shot: create, execute on `stream`, synchronise, check, destroy. */
 int atb_search(atb_handle* h, const atb_params* params, const atb_batch* batch,
