@@ -161,6 +161,7 @@ struct CurveStat {
     int qbits;
     int lobits;
     int qw0;        // the common q_w when uniform_w
+    int qw_min;     // the least q_w
     int uniform_w;  // every q_w equal: the weight words count points
     int thr_unit;   // 1e-15 (the reference's empty-window threshold) is below one
                     // quantised weight unit: "W < 1e-15" is then "W == 0"
@@ -654,6 +655,7 @@ __global__ void __launch_bounds__(kStageBlock) stage_kernel(const StageArgs a) {
         st.lobits = curve_lobits(n);
         st.uniform_w = uniform ? 1 : 0;
         st.qw0 = n > 0 ? qw_max : 0;
+        st.qw_min = n > 0 ? qw_min : 0;
         st.thr_unit = ldexp(1e-15, s_w) < 1.0 ? 1 : 0;
         int ew = 0, ey = 0;
         if (qw_tot > 0) frexp((double)qw_tot, &ew);

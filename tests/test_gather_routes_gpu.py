@@ -130,7 +130,7 @@ def check(engine, kind, wkind, geom, durs=DURS, checked=CHECKED, n=15003, **kw):
         assert count[mine] >= COPIES * len(fill)
     if kind == "flat" and kw.get("n_bins") != 2:  # (two bins have too few windows)
         assert count["given_back"] > 0
-    if kind in ("sampled", "contiguous") and wkind != "point":
+    if kind in ("sampled", "contiguous"):
         assert count["given_back"] == 0
 
 
@@ -193,3 +193,17 @@ def test_unlike_curves_in_one_batch(engine, geom):
     grid = np.concatenate([CHECKED, fillers(geom, N_PER - len(CHECKED), cadence * 15003)])
     count = compare(engine, curves, ws, CHECKED, grid, DURS, config(geom), len(kinds) - 1)
     assert count["counting"] >= 8 * len(grid) / 2 and count["weighted"] >= 8 * len(grid) / 2
+
+
+@pytest.mark.parametrize("decades", [2, 6, 12])
+@pytest.mark.parametrize("geom", ["binned", "fixed"])
+def test_weights_of_many_magnitudes(engine, geom, decades):
+    """The lightest points weigh less than the filter's error, or round to nothing."""
+    cadence = 0.0008 if geom == "binned" else 0.002
+    three = [curve("sampled", 15003 + 64 * i, cadence, 21 + i) for i in range(3)]
+    rng = np.random.default_rng(4)
+    w3 = [(1.0e6 * 10.0 ** -rng.uniform(0, decades, len(c[0]))).astype(np.float32) for c in three]
+    fill = fillers(geom, N_PER - len(CHECKED), max(c[0].max() - c[0].min() for c in three))
+    count = compare(engine, three * 16, w3 * 16, CHECKED, np.concatenate([CHECKED, fill]), DURS,
+                    config(geom))
+    assert count["weighted"] >= 48 * len(fill)
