@@ -746,8 +746,6 @@ __device__ __forceinline__ void team_sync(const Team& tm) {
 struct GroupSmem {
     double tP[kTileP];   // the tile's periods
     int tNB[kTileP];     // and their bin counts
-    int tI[kTileP];      // and their places in the tile
-    int tn;              // how many there are
     double2 PIP[kMaxG];  // (P, 1/P) of each period of the group
     int2 NBB[kMaxG];     // (bin count, histogram offset) of each period
     int fmode[kMaxG];    // fold mode of each period (kFold*)
@@ -763,7 +761,10 @@ struct GroupSmem {
     float den[kMaxWarps];
     int key[kMaxWarps];
     long long tile;
-    long long pb, pe;
+    long long pb;
+    unsigned long long todo;  // the tile's periods still to search: one bit each
+    int np;                   // the tile's periods, those of the gather kernel included
+    int next;                 // first period after the group
     int curve;
     int G;
     int total;
@@ -1857,7 +1858,7 @@ __global__ void __launch_bounds__(NT, MINB) search_kernel(const SearchArgs a) {
                 const int c = a.order[lo];
                 gs.curve = c;
                 gs.pb = tile_start(a, tile, lo, c);
-                gs.pe = min(gs.pb + a.tile_p, a.per_cnt[c]);
+                gs.np = (int)min((long long)a.tile_p, a.per_cnt[c] - gs.pb);
             }
         }
         __syncthreads();
@@ -1875,42 +1876,40 @@ __global__ void __launch_bounds__(NT, MINB) search_kernel(const SearchArgs a) {
             gs.dbins[threadIdx.x] = a.dbins[c * kMaxDur + threadIdx.x];
             gs.dur[threadIdx.x] = a.durations[a.dur_beg[c] + threadIdx.x];
         }
-        // the tile's periods and bin counts, loaded in parallel, without those the
-        // gather kernel searches
+        // the tile's periods and bin counts, loaded in parallel, and a bit for each
+        // that is not the gather kernel's: two ballots by the first warp
         const long long p0 = gs.pb;
-        const int np = (int)(gs.pe - p0);
-        for (int i = threadIdx.x; i < np; i += NT) {
-            const bool mine = !a.scatter || a.scatter[a.flag_off[c] + p0 + i] != 0;
-            int at = i;
-            if (a.scatter) {
-                at = 0;
-                for (int k = 0; k < i; ++k) at += a.scatter[a.flag_off[c] + p0 + k] != 0;
-                if (i == np - 1) gs.tn = at + (mine ? 1 : 0);
-            } else if (i == np - 1) {
-                gs.tn = np;
-            }
-            if (mine) {
-                double P = a.periods[pbeg + p0 + i];
-                if (!(P > 0.0) || !(P < 1.0e300)) {
-                    atomicOr(a.status, 4);
-                    P = 1.0;
-                }
-                gs.tP[at] = P;
-                gs.tI[at] = i;
-                gs.tNB[at] = (GEOM == ATB_GEOM_BINNED)
-                                 ? binned_nbins(P, st.inv_bin_dur, a.oversample, a.max_bins)
-                                 : a.n_bins_fixed;
-            }
+        const int np = gs.np;
+        static_assert(kTileP <= 64 && NT >= kTileP, "one bit and one thread per period");
+        if (threadIdx.x < 32) {
+            const unsigned char* sc = a.scatter ? a.scatter + a.flag_off[c] + p0 : nullptr;
+            const int i = threadIdx.x;
+            const unsigned lo = __ballot_sync(0xffffffffu, i < np && (!sc || sc[i]));
+            const unsigned hi = __ballot_sync(0xffffffffu, 32 + i < np && (!sc || sc[32 + i]));
+            if (i == 0) gs.todo = (unsigned long long)hi << 32 | lo;
         }
         __syncthreads();
-        const int pe = gs.tn;
-        int pn = 0;
-        while (pn < pe) {
+        const unsigned long long todo = gs.todo;
+        if (threadIdx.x < kTileP && (todo >> threadIdx.x & 1ULL)) {
+            const int i = threadIdx.x;
+            double P = a.periods[pbeg + p0 + i];
+            if (!(P > 0.0) || !(P < 1.0e300)) {
+                atomicOr(a.status, 4);
+                P = 1.0;
+            }
+            gs.tP[i] = P;
+            gs.tNB[i] = (GEOM == ATB_GEOM_BINNED)
+                            ? binned_nbins(P, st.inv_bin_dur, a.oversample, a.max_bins)
+                            : a.n_bins_fixed;
+        }
+        __syncthreads();
+        int pn = todo ? __ffsll((long long)todo) - 1 : kTileP;
+        while (pn < kTileP) {
             if (threadIdx.x == 0) {
                 int g = 0, base = 0;
                 int p = pn;
                 double ipmax = 0.0, pmax = 0.0;
-                while (p < pe && g < kMaxG) {
+                while (p < kTileP && g < kMaxG) {
                     const double P = gs.tP[p];
                     const int NB = gs.tNB[p];
                     const int need = NB + 2;
@@ -1920,12 +1919,14 @@ __global__ void __launch_bounds__(NT, MINB) search_kernel(const SearchArgs a) {
                     pmax = max(pmax, P);
                     gs.PIP[g] = make_double2(P, IP);
                     gs.NBB[g] = make_int2(NB, base);
-                    gs.slot[g] = obeg + p0 + gs.tI[p];
+                    gs.slot[g] = obeg + p0 + p;
                     base += need;
                     ++g;
-                    ++p;
+                    const unsigned long long rest = todo & ~(2ULL * (1ULL << p) - 1ULL);
+                    p = rest ? __ffsll((long long)rest) - 1 : kTileP;
                     if (base > a.cap) break;  // a lone oversized period: global histogram
                 }
+                gs.next = p;
                 gs.G = g;
                 gs.total = base;
                 gs.glob = base > a.cap ? 1 : 0;
@@ -1961,7 +1962,7 @@ __global__ void __launch_bounds__(NT, MINB) search_kernel(const SearchArgs a) {
             } else {
                 run_group<GEOM, false>(a, gs, s_hist, st, so, n_pad, nd);
             }
-            pn += gs.G;
+            pn = gs.next;
             __syncthreads();
         }
     }
