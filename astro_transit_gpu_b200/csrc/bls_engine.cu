@@ -84,13 +84,11 @@ constexpr int kMaxDur = 32;            // durations per curve
 // unclamped one) and start + length never overflows an int.
 constexpr int kLenCap = 1 << 28;
 constexpr int kStageAlign = 32;        // staged curves start at multiples of 32 points
-// Threads of a stage CTA (one CTA per curve): kStageBlock for up to kStageWide
-// curves, so that long curves of a small batch are staged in parallel (200 000 points
-// 1.11 -> 0.44 ms, one curve of 15 000 52 -> 41 us); more curves fill the GPU with
-// kStageBlockB each (2000 of 15 000 points: 0.57 against 0.60 ms).
+// Threads of a stage CTA (one CTA per curve), see stage_threads
 constexpr int kStageBlock = 1024;
-constexpr int kStageBlockB = 256;
-constexpr int kStageWide = 592;
+constexpr int kStageBlockM = 512;
+constexpr int kStageBlockS = 256;
+constexpr long long kStageLong = 18000;
 constexpr double kDefaultMergeRun = 8.0;   // atb_params.merge_run = 0
 // atb_params.cta_threads = 0 with fixed bins: four 256-thread CTAs per SM
 // (measured faster than two 512-thread ones for fixed bins; slower for the
@@ -495,8 +493,8 @@ __device__ bool checked_tight_ok(const StageArgs& a, int c, long long n, double*
     return real_bins >= 1.0 && (double)n < kCheckedTightAvg * real_bins;
 }
 
-template <typename YT>
-__global__ void __launch_bounds__(kStageBlock) stage_kernel(const StageArgs a) {
+template <typename YT, int NT>
+__global__ void __launch_bounds__(NT) stage_kernel(const StageArgs a) {
     __shared__ double shd[kStageBlock / 32];
     __shared__ long long shl[kStageBlock / 32];
     const int c = blockIdx.x;
@@ -2223,6 +2221,7 @@ struct atb_plan {
     int y_is_f64 = 0;
     int grid = 0;
     int smem_bytes = 0;
+    int stage_nt = kStageBlock;  // threads per stage CTA
     int nt = kBlock;        // threads per search CTA
     int minb = kMinBlocks;  // resident search CTAs per SM
     long long n_tiles = 0;
@@ -2391,12 +2390,27 @@ bool plan_shape(const atb_params* prm, int* nt, int* minb) {
     return false;
 }
 
+// Threads per stage CTA.  A batch of more points than n_sm curves of its longest
+// length is bound by throughput, and the smallest CTAs waste least (300 curves of
+// 1000 / 15 000 points: 26 / 151 us with 256 threads, 43 / 154 with 512, 89 / 191 with
+// 1024).  In others the longest curve's CTA is the last: 512 threads up to kStageLong
+// points (one curve of 4000 / 15 000 points: 34 / 59 us against 39 / 74 with 256 and 42 / 62
+// with 1024), 1024 beyond (40 000 points: 137 us against 147 with 512 and 216 with 256).
+int stage_threads(int n_sm, long long n_longest, long long n_all) {
+    if (n_all > n_sm * n_longest) return kStageBlockS;
+    return n_longest < kStageLong ? kStageBlockM : kStageBlock;
+}
+
+template <typename YT>
+void stage_launch(int nt, int n_curves, const StageArgs& sa, cudaStream_t s) {
+    if (nt == kStageBlockS) stage_kernel<YT, kStageBlockS><<<n_curves, nt, 0, s>>>(sa);
+    else if (nt == kStageBlockM) stage_kernel<YT, kStageBlockM><<<n_curves, nt, 0, s>>>(sa);
+    else stage_kernel<YT, kStageBlock><<<n_curves, kStageBlock, 0, s>>>(sa);
+}
+
 int launch_stage(atb_plan* p, cudaStream_t s) {
-    const int nt = p->n_curves <= kStageWide ? kStageBlock : kStageBlockB;
-    if (p->y_is_f64)
-        stage_kernel<double><<<p->n_curves, nt, 0, s>>>(p->sa);
-    else
-        stage_kernel<float><<<p->n_curves, nt, 0, s>>>(p->sa);
+    if (p->y_is_f64) stage_launch<double>(p->stage_nt, p->n_curves, p->sa, s);
+    else stage_launch<float>(p->stage_nt, p->n_curves, p->sa, s);
     ATB_CUDA(p->h, cudaGetLastError());
     return ATB_OK;
 }
@@ -2659,12 +2673,13 @@ int plan_create(atb_handle* h, const atb_params* prm, const atb_batch* b, const 
     std::vector<long long> pt_off(nc + 1), t_off(nc), per_beg(nc), per_cnt(nc), dur_beg(nc),
         out_beg(nc), stage_off(nc), tile_off(nc + 1);
     std::vector<int> dur_cnt(nc), order(nc);
-    long long staged = 0, n_out_max = 0;
+    long long staged = 0, n_out_max = 0, n_longest = 0;
     for (int c = 0; c <= nc; ++c) pt_off[c] = b->point_offset[c];
     for (int c = 0; c < nc; ++c) {
         const long long n = pt_off[c + 1] - pt_off[c];
         if (n < 0) return fail(h, ATB_EINVAL, "curve %d: decreasing point_offset", c);
         if (n > (1LL << 26)) return fail(h, ATB_EINVAL, "curve %d: more than 2^26 points", c);
+        n_longest = std::max(n_longest, n);
         t_off[c] = b->time_offset ? b->time_offset[c] : pt_off[c];
         per_beg[c] = b->period_begin[c];
         per_cnt[c] = b->period_count[c];
@@ -2716,6 +2731,7 @@ int plan_create(atb_handle* h, const atb_params* prm, const atb_batch* b, const 
     p->prm = *prm;
     p->n_curves = nc;
     p->y_is_f64 = b->y_is_f64 ? 1 : 0;
+    p->stage_nt = stage_threads(h->n_sm, n_longest, pt_off[nc] - pt_off[0]);
     p->n_tiles = tile_off[nc];
     p->nt = cta_nt;
     p->minb = cta_minb;
@@ -3379,10 +3395,9 @@ extern "C" int atb_search_curve_static(const atb_params* prm, const double* t, c
     sa.geometry = prm->geometry;
     sa.n_bins_fixed = prm->n_bins;
     sa.max_bins = prm->max_bins;
-    if (y_is_f64)
-        stage_kernel<double><<<1, kStageBlock, 0, s>>>(sa);
-    else
-        stage_kernel<float><<<1, kStageBlock, 0, s>>>(sa);
+    // (one size for every n: another would be a kernel that a later call loads)
+    if (y_is_f64) stage_launch<double>(kStageBlockM, 1, sa, s);
+    else stage_launch<float>(kStageBlockM, 1, sa, s);
 
     // Astropy bins: the largest period's bin count and the durations' window
     // lengths in bins (written by the stage kernel).  A period whose
