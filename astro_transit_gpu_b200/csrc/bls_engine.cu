@@ -76,7 +76,10 @@ static_assert(kBlock % 32 == 0 && kBlock / 32 >= 2 && kBlock / 32 <= 32 &&
               "search CTA: a power-of-two number of warps, at most 1024 threads");
 constexpr int kBenchBlock = 512;  // threads of the microbenchmark kernels
 constexpr int kR = ATB_POINTS_PER_THREAD;    // consecutive points a thread holds in registers
-constexpr int kTileP = 64;             // periods per work-queue tile
+constexpr int kTileP = 64;             // periods per work-queue tile, at most
+constexpr int kTileMin = 8;            // and, unless asked for, at least (see plan_create)
+constexpr int kTileMinLong = 4;
+constexpr long long kLongCurve = 60000;
 constexpr int kMaxG = 64;              // periods per shared-memory group
 constexpr int kMaxDur = 32;            // durations per curve
 // Window lengths in bins are clamped to kLenCap: every bin count is below 2^27,
@@ -2707,12 +2710,20 @@ int plan_create(atb_handle* h, const atb_params* prm, const atb_batch* b, const 
     // periods per tile: as requested, else the largest power of two up to
     // kTileP that still gives every resident CTA about four tiles (a small
     // batch -- one curve of a few thousand periods -- otherwise leaves most
-    // SMs idle)
+    // SMs idle), at least kTileMin; kTileMinLong for long curves with astropy bins,
+    // whose longest periods, capped or searched in passes, take up to nine times the
+    // shortest: a tile of eight of them, started first beside another such tile on
+    // its SM, set the whole time (70 403 points, 4172 periods up to 33.5 d, 1999 bins:
+    // 1.58 ms by tiles of 8, 0.84 by 4; shortest first 1.17).  Shorter curves lose by
+    // it: the periods of a tile share the loads of its points (15 000 points, 5000
+    // periods: 147 us by tiles of 8, 158 by 4).
     int tile_p = prm->tile_periods;
     if (tile_p < 1 || tile_p > kTileP) {
         const long long slots = 4LL * h->n_sm * cta_minb;
+        const int least = prm->geometry == ATB_GEOM_BINNED && n_longest >= kLongCurve
+                              ? kTileMinLong : kTileMin;
         tile_p = kTileP;
-        while (tile_p > 8) {
+        while (tile_p > least) {
             long long tiles = 0;
             for (int c = 0; c < nc; ++c) tiles += (per_cnt[c] + tile_p - 1) / tile_p;
             if (tiles >= slots) break;
