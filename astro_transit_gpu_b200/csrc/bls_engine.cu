@@ -98,15 +98,6 @@ constexpr double kDefaultMergeRun = 8.0;   // atb_params.merge_run = 0
 // binned geometry, whose larger histograms want the bigger shared-memory share)
 constexpr int kDefaultFixedThreads = kBlockB;
 constexpr int kChunk = 32 * kR;        // staged points of one warp's fold step
-// cost of one look-up of the prefix-gather search in scattered points (bls_gather.cuh)
-#ifndef ATB_LOOK_COST_BINNED
-#define ATB_LOOK_COST_BINNED 1.1
-#endif
-#ifndef ATB_LOOK_COST_FIXED
-#define ATB_LOOK_COST_FIXED 5.0
-#endif
-constexpr double kLookCostBinned = ATB_LOOK_COST_BINNED;
-constexpr double kLookCostFixed = ATB_LOOK_COST_FIXED;
 constexpr double kMagicSlot = 4503599627370497.0;   // 2^52 + 1: x + C (rz) = 2^52 + int(x) + 1, x in (-1, 2^31 - 1)
 constexpr double kMagicFloor = 6755399441055744.0;  // 1.5*2^52: (m + C)(rd) - C = floor(m), |m| < 2^50
 
@@ -2242,6 +2233,7 @@ struct atb_plan {
         int n_scatter;               // some period is scattered
         int status;
         int nb_max;                  // set-up: the largest bin count
+        GatherPrice price;
     };
     Control* control = nullptr;
     int* status = nullptr;
@@ -2428,12 +2420,12 @@ GatherFn gather_fn(int geom, bool packed) {
 // The search: gathered periods (when the plan has tables), then scattered ones.
 int launch_search(atb_plan* p, cudaStream_t s) {
     if (p->ga.tab) {
-        if (p->prm.geometry == ATB_GEOM_BINNED)
-            table_kernel<ATB_GEOM_BINNED><<<p->n_curves, kTableBlock, 0, s>>>(p->qa, p->ga,
-                                                                             p->tstats);
-        else
-            table_kernel<ATB_GEOM_FIXED><<<p->n_curves, kTableBlock, 0, s>>>(p->qa, p->ga,
-                                                                            p->tstats);
+        const bool binned = p->prm.geometry == ATB_GEOM_BINNED;
+        (binned ? gain_kernel<ATB_GEOM_BINNED> : gain_kernel<ATB_GEOM_FIXED>)
+            <<<p->n_curves, kTableBlock, 0, s>>>(p->qa, p->ga, p->tstats);
+        ATB_CUDA(p->h, cudaGetLastError());
+        (binned ? table_kernel<ATB_GEOM_BINNED> : table_kernel<ATB_GEOM_FIXED>)
+            <<<p->n_curves, kTableBlock, 0, s>>>(p->qa, p->ga, p->tstats);
         ATB_CUDA(p->h, cudaGetLastError());
         for (int w = 0; w < p->ga.vs; ++w) {  // counting curves, then weighted ones
             gather_fn(p->prm.geometry, w == 0)<<<p->gather_grid[w], kGatherBlock, p->gather_smem[w],
@@ -2531,9 +2523,13 @@ int plan_gather(atb_plan* p, const std::vector<long long>& pt_off,
     ga.n_gather = p->control->n_gather;
     ga.n_back = &p->control->n_back;
     ga.n_scatter = &p->control->n_scatter;
-    for (int w = 0; w < ga.vs; ++w)
+    ga.price = &p->control->price;
+    for (int w = 0; w < ga.vs; ++w) {
+        ga.warps[w] = p->h->n_sm * occ[w] * kGatherWarps;
+        ga.one_cta[w] = occ[w] == 1;
         p->gather_grid[w] =
             (int)std::max(1LL, std::min((long long)p->h->n_sm * occ[w], 4 * p->n_tiles));
+    }
     p->ga = ga;
     p->qa.n_scatter = ga.n_scatter;
     return ATB_OK;
@@ -2934,7 +2930,7 @@ int atb_plan_execute(atb_plan* p, void* stream) {
 
 int atb_plan_kernel_count(const atb_plan* p) {
     if (!p) return 0;
-    return 1 + (p->n_tiles > 0 ? (p->ga.tab ? 2 + p->ga.vs : 1) : 0) + (p->best ? 1 : 0);
+    return 1 + (p->n_tiles > 0 ? (p->ga.tab ? 3 + p->ga.vs : 1) : 0) + (p->best ? 1 : 0);
 }
 
 int atb_plan_gathered(atb_plan* p, int64_t* counting, int64_t* weighted, int64_t* given_back) {

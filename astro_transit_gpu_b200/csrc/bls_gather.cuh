@@ -51,10 +51,11 @@ constexpr int kRowPad = 128;                     // columns a block of look-ups 
 constexpr long long kGatherMinPoints = 4096;      // shorter curves search faster than a table is made
 constexpr long long kGatherMaxPoints = (1LL << 18) - 1;
 constexpr long long kGatherMinPeriods = 32;      // of a curve
-// A table pays when what it saves, over the whole GPU, outlasts its making by one CTA (about
-// 7 ns per point, up to 600 curves at a time): in points scattered (0.25 SM clocks each)
-// per point of the curve and curve of the batch.
-constexpr long long kTableLatency = 12000;
+// Prices, in the quarters of an SM clock of gather_gain: a table is made by one CTA, 6 ns per
+// point, while the rest of the GPU waits for it, and by up to 600 CTAs at a time.
+constexpr long long kTableLatency = 12000;       // per point of the longest curve
+constexpr long long kTablePrice = kTableLatency / 600;  // per point of every curve
+constexpr int kPriceClasses = 24;                // curve lengths by quarters of an octave
 constexpr int kHeadMax = 17;                     // saved prefix entries 0..oversample (<= 16)
 
 // cells reserved for a curve of n points (0: too short or too long for a table)
@@ -62,6 +63,22 @@ __host__ __device__ inline long long gather_cells(long long n) {
     return n < kGatherMinPoints || n > kGatherMaxPoints
                ? 0
                : (2 * n + 1024 + kMaxRows * (kRowPad + 16)) / 8 * 8;
+}
+
+// What the curves of one class of lengths (quarters of an octave from kGatherMinPoints)
+// would save and cost, summed over the batch by gain_kernel.
+struct GatherPrice {
+    long long saved[kPriceClasses];   // points scattered, less the look-ups
+    long long looks[kPriceClasses];   // the look-ups alone
+    long long periods[kPriceClasses];
+    long long points[kPriceClasses];
+    int longest[kPriceClasses];
+};
+
+__host__ __device__ inline int price_class(long long n) {
+    int oct = 0;
+    while (n >> (oct + 13)) ++oct;  // 4096..8191: 0
+    return oct * 4 + (int)(n >> (oct + 10) & 3);
 }
 
 // Constants of a curve's windows (and of one fixed-bin period whose trash slot
@@ -97,6 +114,7 @@ struct TableStat : CurveStat {
     int g_colmax;    // last column a look-up may use
     int lmax;        // longest window in bins (astropy bins)
     double g_scale;  // table units (2^-20 cell) per unit time
+    long long n_g;   // periods that are gathered
     GatherConsts gk;
 };
 
@@ -110,37 +128,50 @@ struct GatherArgs {
     unsigned long long* n_gather;  // periods that are gathered, by kernel
     unsigned long long* n_back;    // of these, given back to the scatter kernel
     int* n_scatter;            // some period is scattered
+    GatherPrice* price;
+    int warps[2];              // resident warps of the packed and the weighted kernel,
+    int one_cta[2];            // and whether they are one CTA per SM
     int vs;                    // 2 when weights are given, else 1
     int ring;                  // prefix entries a warp holds
 };
 
-// What gathering a period saves, in scattered points; -INFINITY where it cannot be
-// gathered.  Measured (search kernels, SM clocks per point, look-up and bin): on one-sector
-// curves of 15 000 points and 0.004 d bins scattering takes 0.25 per point and 2.8 per bin
-// (clear, scan, windows), gathering 0.3 per look-up -- whole blocks of 128 per cycle --
-// and 2.3 per bin, so a look-up counts about 1.1 points and a bin saves two; curves
-// whose look-ups are 0.72, 0.9 and 1.01 of their points took 0.85, 0.78 and 1.03 of
-// their scattering time.  Weighted curves (twice the table, four reductions per
-// point) break even at half a look-up per point, fixed bins, whose look-ups
-// take a cache line each, at one for five points (weighted: ten).  A period that does not
-// fit the scatter's shared histogram would fold its points once per bin-range pass.
+// What gathering a period saves, in quarters of an SM clock (about a scattered point of a
+// counting curve); -INFINITY where it cannot be gathered.  `look` receives the look-ups'
+// share.  Fitted to both kernels' times of 340 batches (15 000 to 150 000 points, periods
+// of 0.6 to 150 d, 6 and 8 durations, 0.002 and 0.004 d bins; 592 periods of 32 curves):
+//   astropy bins, counting: scattering 0.23 clocks per point and pass, 3.5 per bin (clear,
+//     scan, windows) and 2.6 per point of the last bin where max_bins cuts the period (they
+//     add to one address); gathering 0.39 per look-up -- whole blocks of 128 per cycle -- and
+//     2.2 per bin; within 20 % of the times.  Weighted: 0.37, 3.7, 3.3; 0.75, 1.9.
+//   fixed bins, whose look-ups take a cache line each: 0.8 to 1.5 per look-up (weighted
+//     2 to 3.3).  One look-up for five points (weighted: ten) breaks even: 15 000 points,
+//     200 bins and 10 cycles scatter in 5500 clocks and gather in 4400; 150 000 points, 300
+//     bins and 40 cycles in 43 000 and 31 000, 119 cycles in 38 500 and 71 400.
+//     Where the prefix entries leave an SM one CTA (from 320 bins, `one_cta`), a period
+//     costs 5 clocks per bin more (weighted 2.5): 500 bins and one cycle of 15 000 points
+//     scatter in 7800 clocks and gather in 8100.
 template <int GEOM>
 __device__ __forceinline__ double gather_gain(const CurveStat& st, int n, int lmax, double P,
-                                              int NB, int os, int cap) {
+                                              int NB, int os, int cap, bool one_cta,
+                                              double& look) {
     // (a period beyond 64 spans would leave the table's number range)
     if (!(P > 0.0) || !(P <= 64.0 * st.dt_absmax)) return -INFINITY;
     const double cycles = floor(st.dt_absmax * (1.0 / P)) + 1.0;
-    double bounds = (double)NB + 1.0, passes = 1.0, bins = 0.0;
+    const bool cnt = st.cnt_win != 0;
     if (GEOM == ATB_GEOM_BINNED) {
         if (NB <= 2 * os) return -INFINITY;  // the padding copy's ranges overlap
-        bounds = fmin(bounds, P * st.inv_bin_dur + 1.0);
-        bins = 2.0 * bounds;
-        if (NB + 2 > cap) passes = ceil((double)NB / (double)max(cap - 2 - lmax, 64));
+        const double bounds = fmin((double)NB + 1.0, P * st.inv_bin_dur + 1.0);
+        // a period that does not fit the scatter's shared histogram folds its points
+        // once per bin-range pass
+        const double passes =
+            NB + 2 > cap ? ceil((double)NB / (double)max(cap - 2 - lmax, 64)) : 1.0;
+        const double cut = fmax(0.0, 1.0 - (double)NB / (P * st.inv_bin_dur));
+        look = (cnt ? 1.54 : 3.0) * cycles * 128.0 * ceil(bounds * (1.0 / 128.0));
+        return (double)n * ((cnt ? 0.92 : 1.49) * passes + (cnt ? 10.4 : 13.3) * cut) +
+               (cnt ? 5.2 : 7.3) * bounds - look;
     }
-    const double looks = cycles * 128.0 * ceil(bounds * (1.0 / 128.0));
-    return (double)n * passes + bins -
-           (GEOM == ATB_GEOM_BINNED ? kLookCostBinned : kLookCostFixed) *
-               (st.cnt_win ? 1.0 : GEOM == ATB_GEOM_BINNED ? 1.6 : 2.0) * looks;
+    look = (cnt ? 5.0 : 10.0) * cycles * 128.0 * ceil(((double)NB + 1.0) * (1.0 / 128.0));
+    return (double)n - look - (one_cta ? (cnt ? 20.0 : 10.0) * (double)NB : 0.0);
 }
 
 // A running sum: packed (counting curves) one word, else weight and flux.
@@ -331,31 +362,133 @@ __device__ __forceinline__ unsigned long long cell_units(double d, double scale)
     return (unsigned long long)(long long)__double2ll_rd(d * scale) + (unsigned long long)kOffHalf;
 }
 
+// Which curves can have a table, which of their periods it would take and what that
+// saves: before any table is made, so that a batch it does not pay for loses no more
+// than this pass over the grids.  One CTA per curve, after the stage kernel.
+template <int GEOM>
+__global__ void __launch_bounds__(kTableBlock) gain_kernel(const SearchArgs a, const GatherArgs ga,
+                                                           TableStat* stats) {
+    __shared__ TableShared sh;
+    const int c = blockIdx.x, tid = threadIdx.x;
+    const long long n = a.pt_off[c + 1] - a.pt_off[c];
+    const long long cells = ga.cell_off[c + 1] - ga.cell_off[c];
+    const long long np = a.per_cnt[c];
+    TableStat sg;
+    static_cast<CurveStat&>(sg) = a.stats[c];
+    const double T = sg.dt_absmax;
+    int lmax = 0;
+    if (GEOM == ATB_GEOM_BINNED)
+        for (int k = 0; k < sg.n_dur; ++k) lmax = max(lmax, a.dbins[c * kMaxDur + k]);
+    // packed words: a flux field that holds twice the absolute total, shifted up to
+    // fill it (the filter converts its top 32 bits)
+    sg.g_guard = min(24, 61 - bitlen64(n) - bitlen64(2 * sg.qy_abs));
+    // split weights need two words per cell
+    bool on = cells > 0 && T > 0.0 && T < 1.0e300 &&
+              (sg.cnt_win ? sg.g_guard >= 0 : ga.vs == 2);
+    if (GEOM == ATB_GEOM_BINNED)
+        on = on && sg.thr_unit && sg.bin_dur > 0.0 && sg.inv_bin_dur < 1.0e300 &&
+             a.oversample < kHeadMax && lmax <= ga.ring - 192 &&
+             // (a period's look-ups are at least T / b, and bin-range passes rarely double
+             // the scattering)
+             T * sg.inv_bin_dur <= 1.36 * (double)n;
+    else
+        on = on && 2 * a.n_bins_fixed + 1 <= ga.ring;
+    unsigned char* scatter = a.scatter + a.flag_off[c];
+    long long n_g = 0, saved = 0, looks = 0;
+    if (on) {
+        const bool one_cta = ga.one_cta[sg.cnt_win ? 0 : 1] != 0;
+        for (long long i = tid; i < np; i += kTableBlock) {
+            const double P = a.periods[a.per_beg[c] + i];
+            const int NB = GEOM == ATB_GEOM_BINNED
+                               ? binned_nbins(P, sg.inv_bin_dur, a.oversample, a.max_bins)
+                               : a.n_bins_fixed;
+            double look = 0.0;
+            const double gain = gather_gain<GEOM>(
+                sg, (int)n, lmax, P, NB, a.oversample, a.cap, one_cta, look);
+            // astropy bins: every period that can be, or none -- the look-ups per point
+            // hardly depend on the period, and a curve split over both kernels took
+            // longer than in either; fixed bins: the periods that gain
+            const bool g = gain > (GEOM == ATB_GEOM_BINNED ? -INFINITY : 0.0);
+            scatter[i] = g ? 0 : 1;
+            n_g += g ? 1 : 0;
+            if (g) {
+                saved += (long long)fmin(gain, 1.0e9);
+                looks += (long long)fmin(look, 1.0e9);
+            }
+        }
+        n_g = tb_sum(n_g, sh);
+        saved = tb_sum(saved, sh);
+        looks = tb_sum(looks, sh);
+        on = n_g > 0 && saved >= kTablePrice * n;
+    }
+    if (!on) {
+        __syncthreads();
+        for (long long i = tid; i < np; i += kTableBlock) scatter[i] = 1;
+    }
+    if (tid == 0) {
+        sg.g_on = on ? 1 : 0;
+        sg.g_n = (int)min(n, (long long)INT_MAX);
+        sg.lmax = lmax;
+        sg.n_g = n_g;
+        sg.g_rows = sg.g_pitch = sg.g_colmax = sg.g_bl = 0;
+        sg.g_scale = 0.0;
+        stats[c] = sg;
+        if (on) {
+            const int k = price_class(n);
+            atomicAdd((unsigned long long*)ga.price->saved + k, (unsigned long long)saved);
+            atomicAdd((unsigned long long*)ga.price->looks + k, (unsigned long long)looks);
+            atomicAdd((unsigned long long*)ga.price->periods + k, (unsigned long long)n_g);
+            atomicAdd((unsigned long long*)ga.price->points + k, (unsigned long long)n);
+            atomicMax(ga.price->longest + k, (int)n);
+        }
+        if (!on || n_g < np) atomicOr(ga.n_scatter, 1);
+    }
+}
+
+// The last class of lengths that gets tables (-1: none): with it, what they save less
+// what they cost is largest.  Too few periods leave warps of the gather kernel idle and
+// their look-ups take as much longer.
+__device__ __forceinline__ int priced_class(const GatherPrice& p, int warps) {
+    long long saved = 0, looks = 0, periods = 0, points = 0;
+    double best = 0.0;
+    int last = -1;
+    for (int k = 0; k < kPriceClasses; ++k) {
+        if (p.periods[k] == 0) continue;
+        saved += p.saved[k];
+        looks += p.looks[k];
+        periods += p.periods[k];
+        points += p.points[k];
+        const double idle = fmax(0.0, (double)warps / (double)periods - 1.0);
+        const double net = (double)saved - (double)looks * idle -
+                           fmax((double)kTableLatency * (double)p.longest[k],
+                                (double)kTablePrice * (double)points);
+        if (net >= best) {
+            best = net;
+            last = k;
+        }
+    }
+    return last;
+}
+
+// The tables of the curves that pay (CTAs of others end at once).
 template <int GEOM>
 __global__ void __launch_bounds__(kTableBlock) table_kernel(const SearchArgs a, const GatherArgs ga,
                                                             TableStat* stats) {
     __shared__ TableShared sh;
     const int c = blockIdx.x, tid = threadIdx.x;
+    if (!stats[c].g_on) return;
+    TableStat sg = stats[c];
+    const CurveStat& st = sg;
     const long long n = a.pt_off[c + 1] - a.pt_off[c];
     const long long so = a.stage_off[c];
     const long long cells = ga.cell_off[c + 1] - ga.cell_off[c];
     const long long np = a.per_cnt[c];
-    const CurveStat st = a.stats[c];
     const long long n_full = st.ilv ? (n + kR - 1) / kR * kR / kChunk * kChunk : 0;
     const double* sdt = a.sdt + so;
     const double T = st.dt_absmax;
-    int lmax = 0;
-    if (GEOM == ATB_GEOM_BINNED)
-        for (int k = 0; k < st.n_dur; ++k) lmax = max(lmax, a.dbins[c * kMaxDur + k]);
-    // split weights need two words per cell
-    bool on = cells > 0 && T > 0.0 && T < 1.0e300 && (st.cnt_win || ga.vs == 2);
-    if (GEOM == ATB_GEOM_BINNED)
-        on = on && st.thr_unit && st.bin_dur > 0.0 && st.inv_bin_dur < 1.0e300 && a.oversample < kHeadMax && lmax <= ga.ring - 192 &&
-             // (the rule below, before any pass over the points: a period's look-ups are at
-             // least T / b, and bin-range passes rarely double the scattering)
-             kLookCostBinned * T * st.inv_bin_dur <= 1.5 * (double)n;
-    else
-        on = on && 2 * a.n_bins_fixed + 1 <= ga.ring;
+    if (tid == 0) sh.flag = price_class(n) <= priced_class(*ga.price, ga.warps[st.cnt_win ? 0 : 1]);
+    __syncthreads();
+    bool on = sh.flag != 0;
     double scale = 0.0;  // units per time
     int rows = 1;
     if (on) {
@@ -390,47 +523,11 @@ __global__ void __launch_bounds__(kTableBlock) table_kernel(const SearchArgs a, 
             on = T * scale / kOffUnits + (double)(rows * (kRowPad + 16)) < (double)cells;
         }
     }
-    // packed words: a flux field that holds twice the absolute total, shifted up to
-    // fill it (the filter converts its top 32 bits)
-    const int guard = min(24, 61 - bitlen64(n) - bitlen64(2 * st.qy_abs));
-    on = on && (!st.cnt_win || guard >= 0);
-    // which periods are gathered
-    unsigned char* scatter = a.scatter + a.flag_off[c];
-    TableStat sg;
-    static_cast<CurveStat&>(sg) = st;
-    sg.g_rows = sg.g_pitch = sg.g_colmax = sg.g_bl = sg.g_guard = 0;
-    sg.g_scale = 0.0;
-    sg.g_on = on ? 1 : 0;
-    sg.g_n = (int)min(n, (long long)INT_MAX);
-    sg.lmax = lmax;
-    long long n_g = 0, saved = 0;
-    if (on) {
-        for (long long i = tid; i < np; i += kTableBlock) {
-            const double P = a.periods[a.per_beg[c] + i];
-            const int NB = GEOM == ATB_GEOM_BINNED
-                               ? binned_nbins(P, st.inv_bin_dur, a.oversample, a.max_bins)
-                               : a.n_bins_fixed;
-            const double gain = gather_gain<GEOM>(st, (int)n, lmax, P, NB, a.oversample, a.cap);
-            // astropy bins: every period that can be, or none -- the look-ups per point
-            // hardly depend on the period, and a curve split over both kernels took
-            // longer than in either; fixed bins: the periods that gain
-            const bool g = gain > (GEOM == ATB_GEOM_BINNED ? -INFINITY : 0.0);
-            scatter[i] = g ? 0 : 1;
-            n_g += g ? 1 : 0;
-            if (g) saved += (long long)fmin(gain, 1.0e12);
-        }
-        n_g = tb_sum(n_g, sh);
-        saved = tb_sum(saved, sh);
-    }
-    // (what was refused above stays refused: a curve without points has no cells to write
-    // to, and its zero savings would meet its zero price)
-    on = on && saved * min(a.n_curves, 600) >= kTableLatency * n;
     if (on) {
         const int bl = bitlen64(n);
         // the padding copy can repeat every point once: counts below 2^(bl + 1), flux
         // sums within twice the absolute total
         sg.g_bl = bl + 1;
-        sg.g_guard = guard;
         const long long c_last = (long long)(cell_units(sdt[staged_pos(n - 1, n_full)], scale) >> kOffBits);
         const int ncol = (int)(c_last / rows) + 3;
         const int pitch = (ncol + (GEOM == ATB_GEOM_BINNED ? kRowPad : 0) + 7) / 8 * 8;
@@ -538,15 +635,14 @@ __global__ void __launch_bounds__(kTableBlock) table_kernel(const SearchArgs a, 
             else gather_consts<false>(sg, curve_total<false>(sg), sg.gk);
         }
     }
-    if (!on) {
-        __syncthreads();
-        for (long long i = tid; i < np; i += kTableBlock) scatter[i] = 1;
-    }
+    __syncthreads();  // (every thread has read stats[c])
+    if (!on)
+        for (long long i = tid; i < np; i += kTableBlock) a.scatter[a.flag_off[c] + i] = 1;
     if (tid == 0) {
         sg.g_on = on ? 1 : 0;
         stats[c] = sg;
-        if (on) atomicAdd(ga.n_gather + (st.cnt_win ? 0 : 1), (unsigned long long)n_g);
-        if (!on || n_g < np) atomicOr(ga.n_scatter, 1);
+        if (on) atomicAdd(ga.n_gather + (st.cnt_win ? 0 : 1), (unsigned long long)sg.n_g);
+        else atomicOr(ga.n_scatter, 1);
     }
 }
 
