@@ -489,6 +489,7 @@ __global__ void __launch_bounds__(kTableBlock) table_kernel(const SearchArgs a, 
     if (tid == 0) sh.flag = price_class(n) <= priced_class(*ga.price, ga.warps[st.cnt_win ? 0 : 1]);
     __syncthreads();
     bool on = sh.flag != 0;
+    const long long most_shared = GEOM == ATB_GEOM_BINNED ? 0 : n / 512;
     double scale = 0.0;  // units per time
     int rows = 1;
     if (on) {
@@ -509,9 +510,15 @@ __global__ void __launch_bounds__(kTableBlock) table_kernel(const SearchArgs a, 
         }
         on = !__syncthreads_or(unsorted);
         int pick = -1;
+        long long close = 0;  // spacings below the chosen width
 #pragma unroll
-        for (int m = kMaxRows - 1; m >= 0; --m)
-            if (tb_sum(cnt[m], sh) <= n / 1024) pick = m;
+        for (int m = kMaxRows - 1; m >= 0; --m) {
+            const long long k = tb_sum(cnt[m], sh);
+            if (k <= n / 1024) {
+                pick = m;
+                close = k;
+            }
+        }
         on = on && pick >= 0;
         if (on) {
             if (GEOM == ATB_GEOM_BINNED) {
@@ -521,6 +528,18 @@ __global__ void __launch_bounds__(kTableBlock) table_kernel(const SearchArgs a, 
                 scale = kOffUnits * (double)n / T * exp2(0.25 * (pick + 1));
             }
             on = T * scale / kOffUnits + (double)(rows * (kRowPad + 16)) < (double)cells;
+        }
+        // Points that share a cell are decided exactly.  With fixed bins a look-up sees
+        // that; with astropy bins every cycle would have to be looked up with every check,
+        // since its boundaries are (64 curves of 15 000 points, one time repeated: 10.5 ms
+        // against 6.0 without it and 7.5 scattered), so such a curve is scattered.
+        if (on && close > 0) {
+            long long shared = 0;
+            for (long long i = tid; i + 1 < n; i += kTableBlock)
+                shared += cell_units(sdt[staged_pos(i, n_full)], scale) >> kOffBits ==
+                                  cell_units(sdt[staged_pos(i + 1, n_full)], scale) >> kOffBits
+                              ? 1 : 0;
+            on = tb_sum(shared, sh) <= most_shared;
         }
     }
     if (on) {
@@ -624,12 +643,7 @@ __global__ void __launch_bounds__(kTableBlock) table_kernel(const SearchArgs a, 
                 }
             }
         }
-        if (multi > n / 512) on = false;
-        // astropy bins: with several points in some cell every cycle is checked
-        if (GEOM == ATB_GEOM_BINNED && multi > 0) {
-            __syncthreads();
-            for (long long k = tid; k < offset_words(bl); k += kTableBlock) bits[k] = 0xffffffffu;
-        }
+        if (multi > most_shared) on = false;  // (spacings just below the cell's width)
         if (tid == 0) {
             if (pk) gather_consts<true>(sg, curve_total<true>(sg), sg.gk);
             else gather_consts<false>(sg, curve_total<false>(sg), sg.gk);

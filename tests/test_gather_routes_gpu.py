@@ -124,7 +124,9 @@ def check(engine, kind, wkind, geom, durs=DURS, checked=CHECKED, n=15003, **kw):
                     np.concatenate([checked, fill]), durs, config(geom, **kw))
     mine, other = (("weighted", "counting") if wkind == "point" else ("counting", "weighted"))
     assert count[other] == 0
-    if geom == "binned":  # a curve's periods are gathered all (but those of few bins) or none
+    if geom == "binned" and kind == "doubled":  # points that share a cell: scattered
+        assert count[mine] == 0
+    elif geom == "binned":  # a curve's periods are gathered all (but those of few bins) or none
         assert count[mine] >= COPIES * (N_PER - 4)
     else:                 # the long periods at least
         assert count[mine] >= COPIES * len(fill)
@@ -193,7 +195,8 @@ def test_unlike_curves_in_one_batch(engine, geom):
     ws = [weights(k, len(c[0])) for c, k in kinds] * 8
     grid = np.concatenate([CHECKED, fillers(geom, N_PER - len(CHECKED), cadence * 15003)])
     count = compare(engine, curves, ws, CHECKED, grid, DURS, config(geom), len(kinds) - 1)
-    assert count["counting"] >= 8 * len(grid) / 2 and count["weighted"] >= 8 * len(grid) / 2
+    assert count["counting"] >= 8 * len(grid) / 2
+    assert count["weighted"] >= 8 * len(grid) / 2
 
 
 @pytest.mark.parametrize("decades", [2, 6, 12])
@@ -208,3 +211,15 @@ def test_weights_of_many_magnitudes(engine, geom, decades):
     count = compare(engine, three * 16, w3 * 16, CHECKED, np.concatenate([CHECKED, fill]), DURS,
                     config(geom))
     assert count["weighted"] >= 48 * len(fill)
+
+
+@pytest.mark.parametrize("wkind", ["uniform", "point"])
+def test_spacings_just_below_a_cell(engine, wkind):
+    """Spacings of 0.99991 cells: a few points share one, which the table finds out late."""
+    n = 15003
+    t = np.arange(n) * (0.0008 * 0.99991)
+    y = (1.0 + np.random.default_rng(1).normal(0.0, 1e-3, n)).astype(np.float32)
+    grid = np.concatenate([CHECKED, fillers("binned", N_PER - len(CHECKED), t[-1])])
+    w = weights(wkind, n)
+    count = compare(engine, [(t, y)] * COPIES, [w] * COPIES, CHECKED, grid, DURS, config("binned"))
+    assert count["counting"] == 0 and count["weighted"] == 0
