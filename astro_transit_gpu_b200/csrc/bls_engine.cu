@@ -154,6 +154,7 @@ struct CurveStat {
     int lobits;
     int qw0;        // the common q_w when uniform_w
     int qw_min;     // the least q_w
+    int flat;       // every flux value is the same
     int uniform_w;  // every q_w equal: the weight words count points
     int thr_unit;   // 1e-15 (the reference's empty-window threshold) is below one
                     // quantised weight unit: "W < 1e-15" is then "W == 0"
@@ -505,11 +506,12 @@ __global__ void __launch_bounds__(NT) stage_kernel(const StageArgs a) {
 
     // pass 1: magnitudes and validity
     double wmax = 0.0, amax = 0.0, tmax = 0.0;
-    int bad = 0;
+    int bad = 0, varied = 0;
     for (long long i = threadIdx.x; i < n; i += (int)blockDim.x) {
         const double wi = w ? (double)w[i] : 1.0;
         const double yi = (double)y[i];
         if (!(wi > 0.0) || !isfinite(wi) || !isfinite(yi) || !isfinite(t[i])) bad = 1;
+        varied |= y[i] != y[0];
         wmax = max(wmax, wi);
         amax = max(amax, fabs(wi * yi));
         tmax = max(tmax, fabs(t[i] - t_start));
@@ -518,6 +520,7 @@ __global__ void __launch_bounds__(NT) stage_kernel(const StageArgs a) {
     amax = block_max_d(amax, shd);
     tmax = block_max_d(tmax, shd);
     if (__syncthreads_or(bad) && threadIdx.x == 0) atomicOr(a.status, 1);
+    varied = __syncthreads_or(varied);
     const int s_w = q_scale(wmax, qbits);
     const int s_a = q_scale(amax, qbits);
 
@@ -648,6 +651,7 @@ __global__ void __launch_bounds__(NT) stage_kernel(const StageArgs a) {
         st.uniform_w = uniform ? 1 : 0;
         st.qw0 = n > 0 ? qw_max : 0;
         st.qw_min = n > 0 ? qw_min : 0;
+        st.flat = varied ? 0 : 1;
         st.thr_unit = ldexp(1e-15, s_w) < 1.0 ? 1 : 0;
         int ew = 0, ey = 0;
         if (qw_tot > 0) frexp((double)qw_tot, &ew);

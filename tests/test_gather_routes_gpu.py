@@ -23,7 +23,7 @@ N_PER = 1600
 CHECKED = np.array([0.9, 1.0, 1.28, 1.999, 2.0, 2.5, 3.71, 5.0, 6.001, 9.13, 12.4, 13.7, 27.0,
                     26.39, 40.0, 0.13, 0.25, 0.5, 0.5004])
 DURS = np.array([0.04, 0.06, 0.08, 0.12, 0.16, 0.20])
-KINDS = ["sampled", "contiguous", "grid", "doubled", "flat", "plateaus", "flare"]
+KINDS = ["sampled", "contiguous", "grid", "doubled", "flat", "plateaus", "flare", "spike"]
 
 
 @pytest.fixture(scope="module")
@@ -42,7 +42,7 @@ def config(geom, **kw):
 
 def curve(kind, n, cadence, seed):
     rng = np.random.default_rng(seed)
-    if kind == "grid":  # times and bins are multiples of one step
+    if kind in ("grid", "spike"):  # times and bins are multiples of one step
         t = np.arange(n) * cadence
     else:
         g = np.arange(n + n // 10) * cadence + 1400.0
@@ -57,6 +57,9 @@ def curve(kind, n, cadence, seed):
         y[:] = 1.0
     if kind == "plateaus":
         y = R.inject_box(t, np.ones(n), 2.5, t[0] + 0.7, 0.2, 1e-2)
+    if kind == "spike":  # equal but for one point: windows tie by the hundred
+        y[:] = 1.0
+        y[n // 3] += 1e-3
     if kind == "flare":
         y[700:704] += 5.0
     return t, y.astype(np.float32)
@@ -124,16 +127,16 @@ def check(engine, kind, wkind, geom, durs=DURS, checked=CHECKED, n=15003, **kw):
                     np.concatenate([checked, fill]), durs, config(geom, **kw))
     mine, other = (("weighted", "counting") if wkind == "point" else ("counting", "weighted"))
     assert count[other] == 0
-    if geom == "binned" and kind == "doubled":  # points that share a cell: scattered
-        assert count[mine] == 0
+    if kind == "flat" or (geom == "binned" and kind == "doubled"):
+        assert count[mine] == 0  # every window equal; points that share a cell
     elif geom == "binned":  # a curve's periods are gathered all (but those of few bins) or none
         assert count[mine] >= COPIES * (N_PER - 4)
     else:                 # the long periods at least
         assert count[mine] >= COPIES * len(fill)
-    if kind == "flat" and kw.get("n_bins") != 2:  # (two bins have too few windows)
-        assert count["given_back"] > 0
     if kind in ("sampled", "contiguous"):
         assert count["given_back"] == 0
+    if kind == "spike" and geom == "binned" and wkind != "point":
+        assert count["given_back"] > 0
 
 
 @pytest.mark.parametrize("wkind", ["uniform", "point", None])
