@@ -142,7 +142,8 @@ struct GatherArgs {
 //   astropy bins, counting: scattering 0.23 clocks per point and pass, 3.5 per bin (clear,
 //     scan, windows) and 2.6 per point of the last bin where max_bins cuts the period (they
 //     add to one address); gathering 0.39 per look-up -- whole blocks of 128 per cycle -- and
-//     2.2 per bin; within 20 % of the times.  Weighted: 0.37, 3.7, 3.3; 0.75, 1.9.
+//     2.2 per bin; within 20 % of the times.  Weighted: 0.37, 3.7, 3.3; 0.75, 1.9 and
+//     a few hundred per period.
 //   fixed bins, whose look-ups take a cache line each: 0.8 to 1.5 per look-up (weighted
 //     2 to 3.3).  One look-up for five points (weighted: ten) breaks even: 15 000 points,
 //     200 bins and 10 cycles scatter in 5500 clocks and gather in 4400; 150 000 points, 300
@@ -168,7 +169,7 @@ __device__ __forceinline__ double gather_gain(const CurveStat& st, int n, int lm
         const double cut = fmax(0.0, 1.0 - (double)NB / (P * st.inv_bin_dur));
         look = (cnt ? 1.54 : 3.0) * cycles * 128.0 * ceil(bounds * (1.0 / 128.0));
         return (double)n * ((cnt ? 0.92 : 1.49) * passes + (cnt ? 10.4 : 13.3) * cut) +
-               (cnt ? 5.2 : 7.3) * bounds - look;
+               (cnt ? 5.2 : 7.3) * bounds - look - (cnt ? 0.0 : 1500.0);
     }
     look = (cnt ? 5.0 : 10.0) * cycles * 128.0 * ceil(((double)NB + 1.0) * (1.0 / 128.0));
     return (double)n - look - (one_cta ? (cnt ? 20.0 : 10.0) * (double)NB : 0.0);
