@@ -66,7 +66,6 @@ E2E_PARTS = 8  # runs of curves (and streams) of the end-to-end step
 # histogram word layout the stage kernel chose for the curve
 LAYOUT_WORDS = {0: 4, 1: 3, 2: 2, 3: 2}  # split, count, tight, tight (checked)
 LAYOUT_NAMES = {0: "split", 1: "count", 2: "tight", 3: "tight_checked"}
-U64_BYTES_PER_FOLD = 16  # two 8-byte accumulations per update in a 64-bit design
 
 
 def parse(argv=None):
@@ -644,8 +643,11 @@ def main(argv=None):
     red_bytes = float(4.0 * (words * upd).sum())
     achieved = red_bytes / (ms_search * 1e-3) / 1e9
     peak = 4.0 * peaks["smem_red_u32_per_s"] / 1e9
-    ach64 = U64_BYTES_PER_FOLD * u_fold / (ms_search * 1e-3) / 1e9
-    peak64 = 8.0 * peaks["smem_red_u64_per_s"] / 1e9
+    g = plan.gathered()  # of the last profiled execution
+    n_per = sum(len(curve_periods(periods, c)) for c in range(nc))
+    gathered = (g["counting"] + g["weighted"] - g["given_back"]) / max(n_per, 1)
+    lookups = (sum(table_lookups(t[c], curve_periods(periods, c), curve_periods(durs, c))
+                   for c in range(nc)) if gathered == 1.0 and args.method == "parity" else None)
     layout_share = {LAYOUT_NAMES[k]: float(upd[layout == k].sum() / u_fold)
                     for k in LAYOUT_NAMES}
 
@@ -665,26 +667,14 @@ def main(argv=None):
                 "gpu_launches": psess.kernel_count * args.steps},
         "gpu_launches": plan.kernel_count * args.steps,
         "roofline": {
-            "bound": "smem",
-            "kernel": "search_kernel<FIXED>" if args.method == "fast" else "search_kernel<BINNED>",
-            "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
-            "traffic": None,
-            "traffic_source": "no capture of this launch: the committed ones are of the scatter "
-                              "kernel alone",
-            "units": "4 B per 32-bit shared-memory reduction of the scattered form of the search, "
-                     "whether the engine scattered or gathered the curve (gathered curves issue "
-                     "table look-ups instead): 2, 3 or 4 per "
-                     "(point, period) update by the curve's histogram layout (tight, count, "
-                     f"split; a checked tight period that is folded again counts 2); "
-                     f"{u_fold:.3e} updates and {red_bytes / 4:.3e} reductions per launch",
+            **search_roofline(args.workload, args.method, nc, gathered, lookups, ms_search,
+                              achieved, peak,
+                              search_algorithmic_bytes(lens, [len(curve_periods(periods, c))
+                                                              for c in range(nc)])),
             "layout_share_of_updates": layout_share,
-            "peak_source": "atb_bench_smem_red_u32 (conflict-free 32-bit shared-memory "
-                           "reductions, measured live on this GPU)",
             "ms_search": ms_search, "ms_stage": ms_stage,
             "fold_updates_per_s": u_fold / (ms_search * 1e-3),
-            "u64_design": {"achieved": ach64, "peak": peak64, "frac": ach64 / peak64,
-                           "units": "16 B per update (two 64-bit accumulations), against "
-                                    "conflict-free 64-bit shared-memory reductions"},
+            "updates_per_launch": u_fold, "reductions_per_launch_if_scattered": red_bytes / 4,
             "dfma_peak_per_s": peaks["dfma_per_s"],
             "smem_red_u32_random_per_s": peaks["smem_red_u32_random_per_s"],
             "smem_red_u64_random_per_s": peaks["smem_red_u64_random_per_s"],
@@ -801,6 +791,44 @@ class ClockSampler:
         return {"sm_mhz": float(np.median(sm)) if sm else None,
                 "sm_max_mhz": max(mx) if mx else None, "reasons": reasons,
                 "samples": len(self.rows)}
+
+
+def table_lookups(t, periods, durations, oversample=10):
+    """Table look-ups of a gathered curve with uncapped astropy bins: whole rows
+    of 128 boundaries for each cycle of each period."""
+    span = float(np.max(t) - np.min(t))
+    per = np.asarray(periods, np.float64)
+    bounds = np.floor(per / (float(np.min(durations)) / oversample)) + 1.0
+    return float(((np.floor(span / per) + 1.0) * 128.0 * np.ceil(bounds / 128.0)).sum())
+
+
+def search_roofline(workload, method, n_curves, gathered, lookups, ms_search, achieved, peak,
+                    algo_bytes):
+    """What the search is measured against.  Scattered periods are bound by
+    shared-memory reductions, `achieved` of `peak` GB/s.  Gathered ones (a share
+    `gathered` of the batch's) issue none: they are bound by instructions
+    and look-up latency, and no rate of this GPU is their peak."""
+    geom = "<FIXED>" if method == "fast" else "<BINNED>"
+    if gathered == 0.0:
+        return {"bound": "smem", "kernel": "search_kernel" + geom, "achieved": achieved,
+                "peak": peak, "unit": "GB/s", "frac": achieved / peak, "gathered_share": 0.0,
+                "traffic": measured_traffic(workload, method, n_curves, algo_bytes),
+                "traffic_source": "ncu capture of a smaller launch of this workload under "
+                                  "profiles/, scaled to this launch (null: no capture)",
+                "units": "4 B per 32-bit shared-memory reduction the fold issues: 2, 3 or 4 per "
+                         "(point, period) update by the curve's histogram layout (tight, count, "
+                         "split; a checked tight period that is folded again counts 2)",
+                "peak_source": "atb_bench_smem_red_u32 (conflict-free 32-bit shared-memory "
+                               "reductions, measured live on this GPU)"}
+    return {"bound": "issue",
+            "kernel": "gather_kernel" + geom + ("" if gathered == 1.0 else " and search_kernel" + geom),
+            "achieved": None if lookups is None else lookups / (ms_search * 1e-3) / 1e9,
+            "peak": None, "unit": "1e9 table look-ups/s", "frac": None, "gathered_share": gathered,
+            "traffic": None,
+            "traffic_source": "no capture of this launch: the committed ones are of smaller "
+                              "launches of either kernel",
+            "units": "table look-ups of whole rows of 128 boundaries per cycle and period "
+                     "(null: part of the batch is scattered, or fixed bins)"}
 
 
 def search_algorithmic_bytes(lens, counts):
