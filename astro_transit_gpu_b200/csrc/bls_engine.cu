@@ -86,6 +86,7 @@ constexpr int kMaxDur = 32;            // durations per curve
 // so a clamped window never fits a period (it is skipped exactly as the
 // unclamped one) and start + length never overflows an int.
 constexpr int kLenCap = 1 << 28;
+constexpr size_t kTableFree = 256ull << 20;  // look-up tables up to this size are made without asking
 constexpr int kStageAlign = 32;        // staged curves start at multiples of 32 points
 // Threads of a stage CTA (one CTA per curve), see stage_threads
 constexpr int kStageBlock = 1024;
@@ -2225,6 +2226,7 @@ struct atb_plan {
     long long n_tiles = 0;
     std::vector<void*> allocs;
     long long scratch_bytes = 0;
+    long long table_bytes = 0;  // of these, the gather search's
     StageArgs sa{};
     SearchArgs qa{};
     int* best = nullptr;
@@ -2442,9 +2444,25 @@ int launch_search(atb_plan* p, cudaStream_t s) {
     return ATB_OK;
 }
 
-// Tables and launch shape of the gather kernel.  Without memory for the
-// tables, or where they would take more than `limit` bytes (negative: no limit), the
-// plan scatters every period.
+// Device memory a plan could still get: the device's free bytes and, for a
+// stream-ordered plan, what its pool holds unused.
+size_t free_bytes(const atb_plan* p) {
+    size_t free = 0, total = 0;
+    if (cudaMemGetInfo(&free, &total) != cudaSuccess) return 0;
+    unsigned long long held = 0, used = 0;
+    if (p->async && p->h->pool &&
+        cudaMemPoolGetAttribute(p->h->pool, cudaMemPoolAttrReservedMemCurrent, &held) ==
+            cudaSuccess &&
+        cudaMemPoolGetAttribute(p->h->pool, cudaMemPoolAttrUsedMemCurrent, &used) == cudaSuccess)
+        free += held - std::min(held, used);
+    return free;
+}
+
+// Tables and launch shape of the gather kernel.  Without memory for the tables, or where
+// they would take more than `limit` bytes, the plan scatters every period.  Negative: no
+// limit but that tables above kTableFree leave three quarters of the free memory to whoever
+// asks next (they take more than the curves themselves, 40 to 88 bytes per point, and the
+// batches of before they were made filled the device with less).
 int plan_gather(atb_plan* p, const std::vector<long long>& pt_off,
                 const std::vector<long long>& per_cnt, bool weighted, long long limit) {
     if (limit == 0) return ATB_OK;
@@ -2508,6 +2526,7 @@ int plan_gather(atb_plan* p, const std::vector<long long>& pt_off,
     unsigned char* flags = nullptr;
     arr.scratch(&flags, (size_t)flag_off[nc]);
     if (limit > 0 && arr.bytes > (size_t)limit) return ATB_OK;
+    if (limit < 0 && arr.bytes > kTableFree && arr.bytes > free_bytes(p) / 4) return ATB_OK;
     const size_t held = p->allocs.size();
     const long long held_bytes = p->scratch_bytes;
     if (arr.commit(p)) {  // give back what it did get
@@ -2540,6 +2559,7 @@ int plan_gather(atb_plan* p, const std::vector<long long>& pt_off,
     }
     p->ga = ga;
     p->qa.n_scatter = ga.n_scatter;
+    p->table_bytes = p->scratch_bytes - held_bytes;
     return ATB_OK;
 }
 
@@ -2955,6 +2975,7 @@ int atb_plan_gathered(atb_plan* p, int64_t* counting, int64_t* weighted, int64_t
 }
 
 int64_t atb_plan_scratch_bytes(const atb_plan* p) { return p ? p->scratch_bytes : 0; }
+int64_t atb_plan_table_bytes(const atb_plan* p) { return p ? p->table_bytes : 0; }
 
 int atb_plan_curve_layout(atb_plan* p, int32_t* layout, int32_t* occupancy_bits) {
     if (!p || !layout || !occupancy_bits) return ATB_EINVAL;

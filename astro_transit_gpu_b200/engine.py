@@ -262,6 +262,11 @@ class SearchPlan:
     def scratch_bytes(self) -> int:
         return int(self._lib.atb_plan_scratch_bytes(self.ptr))
 
+    @property
+    def table_bytes(self) -> int:
+        """Bytes of `scratch_bytes` in look-up tables."""
+        return int(self._lib.atb_plan_table_bytes(self.ptr))
+
     def execute(self, stream: Optional[torch.cuda.Stream] = None) -> None:
         s = stream if stream is not None else (
             self.stream or torch.cuda.current_stream(self.batch.device))

@@ -128,21 +128,25 @@ def check_request(t: np.ndarray, y: np.ndarray, dy, periods: np.ndarray,
 
 
 def request_bytes(n_points: int, n_periods: int, n_durations: int) -> int:
-    """Device bytes a request holds while its batch runs: inputs (t f64, y, w
+    """Device bytes a request needs while its batch runs: inputs (t f64, y, w
     f32), staged points (16 B), the grids and the per-period outputs (28 B),
-    rounded up for the plan's descriptors; curves of 4096 to 2^18 - 1 points also
-    the look-up table (two cells of 36 B and 16 B of offset bits per point, 2176
-    cells more per curve, a flag per period)."""
-    table = 0
-    if 4096 <= n_points < 1 << 18 and n_periods >= 32:
-        table = n_points * (2 * 36 + 16) + 2176 * 36 + n_periods
-    return int(n_points * (16 + 16) + n_periods * (8 + 28) + n_durations * 8 + 4096 + table)
+    rounded up for the plan's descriptors.  The look-up tables that a batch of
+    dense curves may have beyond these come out of `spare_bytes`."""
+    return int(n_points * (16 + 16) + n_periods * (8 + 28) + n_durations * 8 + 4096)
+
+
+def spare_bytes(budget: int, held: int, pending) -> int:
+    """Bytes of the budget a batch may take for look-up tables, which only make
+    it faster: half of what the running batches and the waiting requests leave,
+    so that the requests that come next are still admitted."""
+    return max(0, budget - held - sum(r.nbytes for r in pending)) // 2
 
 
 class BLSServer:
     """Continuous-batching BLS server (one GPU, one worker thread).
 
-    memory_budget  device bytes the in-flight batches may hold (admission)
+    memory_budget  device bytes the in-flight batches may hold (admission; look-up
+                   tables take only what no waiting request needs)
     max_batch      most requests in one batch
     n_streams      batches in flight at once
     """
@@ -290,7 +294,9 @@ class BLSServer:
                 periods=[r.periods for r in reqs], durations=[r.durations for r in reqs],
                 device=self.device, flux_dtype=reqs[0].flux_dtype,
                 weights=[r.w for r in reqs] if reqs[0].w is not None else None)
-            plan = self.engine.plan(batch, reqs[0].config, stream=stream)
+            with self._cv:
+                spare = spare_bytes(self.memory_budget, self._held, self._pending)
+            plan = self.engine.plan(batch, reqs[0].config, stream=stream, table_bytes=spare)
             plan.execute(stream)
             # outputs back to pinned host memory in the batch's stream order, so
             # the worker only slices them once the batch's event has fired
@@ -300,7 +306,11 @@ class BLSServer:
                 host_out[k].copy_(v, non_blocking=True)
             ev = torch.cuda.Event()
             ev.record(stream)
-        return _Batch(reqs, batch, plan, stream, ev, sum(r.nbytes for r in reqs), host_out)
+        with self._cv:  # (given back with the requests' own bytes)
+            self._held += plan.table_bytes
+            self._max_held = max(self._max_held, self._held)
+        return _Batch(reqs, batch, plan, stream, ev,
+                      sum(r.nbytes for r in reqs) + plan.table_bytes, host_out)
 
     def _finish(self, b: _Batch) -> None:
         try:

@@ -154,7 +154,8 @@ int atb_plan_create_async(atb_handle* h, const atb_params* params, const atb_bat
  * searched by look-ups in per-curve tables, 40 to 88 bytes per point of
  * scratch; a plan whose tables would take more than table_bytes makes none
  * and searches every period with shared-memory histograms.  0 = no tables,
- * negative = no limit.
+ * negative = no limit (as the other plans: tables above 256 MiB take no more
+ * than a quarter of the device's free memory).
  */
 int atb_plan_create_limited(atb_handle* h, const atb_params* params, const atb_batch* batch,
                             const atb_outputs* outputs, void* stream, int64_t table_bytes,
@@ -167,6 +168,8 @@ int atb_plan_check(atb_plan* p);
 int atb_plan_kernel_count(const atb_plan* p);
 /* Bytes of device scratch the plan holds. */
 int64_t atb_plan_scratch_bytes(const atb_plan* p);
+/* Of these, the bytes of its look-up tables (0: every period is searched with histograms). */
+int64_t atb_plan_table_bytes(const atb_plan* p);
 void atb_plan_destroy(atb_plan* p);
 
 /*
