@@ -24,6 +24,7 @@ from dataclasses import dataclass, field
 from typing import Any, Dict, List, Optional, Sequence
 
 import numpy as np
+import torch
 
 from .engine import BLSEngine, CurveBatch, SearchConfig, is_shared_grid, split_outputs
 from .gpu_bls import get_top_k_candidates
@@ -189,7 +190,8 @@ def power_batch(times: Sequence[np.ndarray], fluxes: Sequence[np.ndarray],
                                    periods=checked_p if per_curve_p else checked_p[0],
                                    durations=checked_d if per_curve_d else checked_d[0],
                                    flux_dtype=fdt)
-    plan = BLSEngine.get().plan(batch, cfg)
+    # (stream-ordered: scratch from the engine's pool, not mapped for every call)
+    plan = BLSEngine.get().plan(batch, cfg, stream=torch.cuda.current_stream(batch.device))
     try:
         plan.execute()
         plan.check()

@@ -496,7 +496,9 @@ class BLSEngine:
         with torch.cuda.stream(s):
             key = torch.zeros(nc, dtype=torch.int64, device=batch.device)
             best = torch.empty(nc, dtype=torch.int32, device=batch.device)
-        plan = self.plan(batch, config, {"best_key": key, "best_period": best})
+        # (stream-ordered: a plan of device-wide allocations maps and unmaps its memory
+        # on every call, and waits for other streams' work)
+        plan = self.plan(batch, config, {"best_key": key, "best_period": best}, stream=s)
         try:
             plan.execute(s)
             plan.check()
