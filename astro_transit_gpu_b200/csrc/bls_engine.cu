@@ -92,6 +92,7 @@ constexpr int kStageAlign = 32;        // staged curves start at multiples of 32
 constexpr int kStageBlock = 1024;
 constexpr int kStageBlockM = 512;
 constexpr int kStageBlockS = 256;
+constexpr long long kStageShort = 6000;
 constexpr long long kStageLong = 18000;
 constexpr double kDefaultMergeRun = 8.0;   // atb_params.merge_run = 0
 // atb_params.cta_threads = 0 with fixed bins: four 256-thread CTAs per SM
@@ -359,7 +360,8 @@ __device__ __forceinline__ long long warp_sum(long long v) {
     return v;
 }
 
-// block reductions for the stage kernel (at most kStageBlock threads)
+// block reductions for the stage kernel (NT threads)
+template <int NT>
 __device__ double block_max_d(double v, double* sh) {
     v = warp_max(v);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -367,10 +369,11 @@ __device__ double block_max_d(double v, double* sh) {
     if (lane == 0) sh[warp] = v;
     __syncthreads();
     double r = sh[0];
-    for (int i = 1; i < (int)blockDim.x / 32; ++i) r = max(r, sh[i]);
+    for (int i = 1; i < NT / 32; ++i) r = max(r, sh[i]);
     return r;
 }
 
+template <int NT>
 __device__ long long block_sum_ll(long long v, long long* sh) {
     v = warp_sum(v);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -378,7 +381,7 @@ __device__ long long block_sum_ll(long long v, long long* sh) {
     if (lane == 0) sh[warp] = v;
     __syncthreads();
     long long r = 0;
-    for (int i = 0; i < (int)blockDim.x / 32; ++i) r += sh[i];
+    for (int i = 0; i < NT / 32; ++i) r += sh[i];
     return r;
 }
 
@@ -393,25 +396,26 @@ __device__ long long block_sum_ll(long long v, long long* sh) {
 // (astropy-binned: min(duration)/oversample; fixed: P_max/n_bins), widened by a
 // relative 1e-6 for rounding.  Requires time-ordered points and, for
 // astropy bins, a bin cap (max_bins) that no period of the grid reaches.
+template <int NT>
 __device__ int occupancy_bits(const StageArgs& a, int c, const double* t, long long n, double* shd,
                               long long* shl) {
     // time order
     int unsorted = 0;
-    for (long long i = threadIdx.x; i + 1 < n; i += (int)blockDim.x) unsorted |= t[i] > t[i + 1];
+    for (long long i = threadIdx.x; i + 1 < n; i += NT) unsorted |= t[i] > t[i + 1];
     if (__syncthreads_or(unsorted)) return 64;
     // grid extremes
     const double* per = a.periods + a.per_beg[c];
     const long long np = a.per_cnt[c];
     double pmax = 0.0, pinv = 0.0;
-    for (long long i = threadIdx.x; i < np; i += (int)blockDim.x) {
+    for (long long i = threadIdx.x; i < np; i += NT) {
         const double P = per[i];
         if (P > 0.0 && P < 1.0e300) {
             pmax = max(pmax, P);
             pinv = max(pinv, 1.0 / P);
         }
     }
-    pmax = block_max_d(pmax, shd);
-    pinv = block_max_d(pinv, shd);
+    pmax = block_max_d<NT>(pmax, shd);
+    pinv = block_max_d<NT>(pinv, shd);
     if (!(pinv > 0.0)) return 64;
     double width;
     if (a.geometry == ATB_GEOM_BINNED) {
@@ -431,7 +435,7 @@ __device__ int occupancy_bits(const StageArgs& a, int c, const double* t, long l
     if (!(width > 0.0) || !isfinite(width)) return 64;
     width = width * (1.0 + 1e-6) + 1e-12;
     // K: each thread scans a contiguous range of window starts with a second pointer
-    const long long per_thr = (n + (int)blockDim.x - 1) / (int)blockDim.x;
+    const long long per_thr = (n + NT - 1) / NT;
     const long long i0 = min(n, (long long)threadIdx.x * per_thr);
     const long long i1 = min(n, i0 + per_thr);
     long long kmax = 0;
@@ -447,7 +451,7 @@ __device__ int occupancy_bits(const StageArgs& a, int c, const double* t, long l
             kmax = max(kmax, j - i);
         }
     }
-    kmax = (long long)block_max_d((double)kmax, shd);
+    kmax = (long long)block_max_d<NT>((double)kmax, shd);
     const double span = n > 0 ? t[n - 1] - t[0] : 0.0;
     const double cycles = floor(span * pinv * (1.0 + 1e-9)) + 3.0;
     const double m = cycles * (double)kmax;
@@ -461,19 +465,20 @@ __device__ int occupancy_bits(const StageArgs& a, int c, const double* t, long l
 // and, for astropy bins, a bin cap (max_bins) that no period reaches (the cap
 // piles points into the last bin).  Bins far fuller than the average only cost
 // a second fold of their period.
+template <int NT>
 __device__ bool checked_tight_ok(const StageArgs& a, int c, long long n, double* shd) {
     const double* per = a.periods + a.per_beg[c];
     const long long np = a.per_cnt[c];
     double pmax = 0.0, pinv = 0.0;
-    for (long long i = threadIdx.x; i < np; i += (int)blockDim.x) {
+    for (long long i = threadIdx.x; i < np; i += NT) {
         const double P = per[i];
         if (P > 0.0 && P < 1.0e300) {
             pmax = max(pmax, P);
             pinv = max(pinv, 1.0 / P);
         }
     }
-    pmax = block_max_d(pmax, shd);
-    pinv = block_max_d(pinv, shd);
+    pmax = block_max_d<NT>(pmax, shd);
+    pinv = block_max_d<NT>(pinv, shd);
     if (!(pinv > 0.0)) return false;
     double real_bins = (double)a.n_bins_fixed;
     if (a.geometry == ATB_GEOM_BINNED) {
@@ -491,8 +496,8 @@ __device__ bool checked_tight_ok(const StageArgs& a, int c, long long n, double*
 
 template <typename YT, int NT>
 __global__ void __launch_bounds__(NT) stage_kernel(const StageArgs a) {
-    __shared__ double shd[kStageBlock / 32];
-    __shared__ long long shl[kStageBlock / 32];
+    __shared__ double shd[NT / 32];
+    __shared__ long long shl[NT / 32];
     const int c = blockIdx.x;
     const long long p0 = a.pt_off[c];
     const long long n = a.pt_off[c + 1] - p0;
@@ -507,21 +512,29 @@ __global__ void __launch_bounds__(NT) stage_kernel(const StageArgs a) {
 
     // pass 1: magnitudes and validity
     double wmax = 0.0, amax = 0.0, tmax = 0.0;
-    int bad = 0, varied = 0;
-    for (long long i = threadIdx.x; i < n; i += (int)blockDim.x) {
+    int bad = 0;
+    for (long long i = threadIdx.x; i < n; i += NT) {
         const double wi = w ? (double)w[i] : 1.0;
         const double yi = (double)y[i];
         if (!(wi > 0.0) || !isfinite(wi) || !isfinite(yi) || !isfinite(t[i])) bad = 1;
-        varied |= y[i] != y[0];
         wmax = max(wmax, wi);
         amax = max(amax, fabs(wi * yi));
         tmax = max(tmax, fabs(t[i] - t_start));
     }
-    wmax = block_max_d(wmax, shd);
-    amax = block_max_d(amax, shd);
-    tmax = block_max_d(tmax, shd);
+    wmax = block_max_d<NT>(wmax, shd);
+    amax = block_max_d<NT>(amax, shd);
+    tmax = block_max_d<NT>(tmax, shd);
     if (__syncthreads_or(bad) && threadIdx.x == 0) atomicOr(a.status, 1);
-    varied = __syncthreads_or(varied);
+    // A flat curve?  (Apart from pass 1, whose loads one more comparison kept from running
+    // ahead: 153 curves of 46 942 points, 256 threads, 532 us instead of 389.  The first
+    // block of points answers it for any other curve.)
+    int varied = 0;
+    for (long long i0 = threadIdx.x; __syncthreads_or(i0 < n) && !varied; i0 += 8 * NT) {
+        int v = 0;
+#pragma unroll
+        for (int k = 0; k < 8; ++k) v |= i0 + k * NT < n && y[i0 + k * NT] != y[0];
+        varied = __syncthreads_or(v);
+    }
     const int s_w = q_scale(wmax, qbits);
     const int s_a = q_scale(amax, qbits);
 
@@ -529,7 +542,7 @@ __global__ void __launch_bounds__(NT) stage_kernel(const StageArgs a) {
     // range of the quantised weights decides the histogram layout
     long long sqw = 0, sqa = 0;
     int qw_min = 0x7fffffff, qw_max = -1;
-    for (long long i = threadIdx.x; i < n; i += (int)blockDim.x) {
+    for (long long i = threadIdx.x; i < n; i += NT) {
         const double wi = w ? (double)w[i] : 1.0;
         const double yi = (double)y[i];
         const long long qa = __double2ll_rn(ldexp(wi, s_w));
@@ -538,19 +551,19 @@ __global__ void __launch_bounds__(NT) stage_kernel(const StageArgs a) {
         qw_min = min(qw_min, (int)qa);
         qw_max = max(qw_max, (int)qa);
     }
-    sqw = block_sum_ll(sqw, shl);
-    sqa = block_sum_ll(sqa, shl);
-    qw_max = (int)block_max_d((double)qw_max, shd);
-    qw_min = -(int)block_max_d(-(double)qw_min, shd);
+    sqw = block_sum_ll<NT>(sqw, shl);
+    sqa = block_sum_ll<NT>(sqa, shl);
+    qw_max = (int)block_max_d<NT>((double)qw_max, shd);
+    qw_min = -(int)block_max_d<NT>(-(double)qw_min, shd);
     const bool uniform = n > 0 && qw_min == qw_max;
     int packmode = uniform ? kPackCount : kPackSplit;
     int tight_bits = 64;
-    if (uniform && a.periods) tight_bits = occupancy_bits(a, c, t, n, shd, shl);
+    if (uniform && a.periods) tight_bits = occupancy_bits<NT>(a, c, t, n, shd, shl);
     if (uniform && tight_bits <= kTightMaxBits && qbits <= 27) packmode = kPackTight;
     // no proven bound: the checked tight layout where bins are sparse on average
     bool tcheck = false;
     if (uniform && packmode != kPackTight && a.periods && qbits <= 27 && n < (1LL << 24) &&
-        checked_tight_ok(a, c, n, shd)) {
+        checked_tight_ok<NT>(a, c, n, shd)) {
         packmode = kPackTight;
         tight_bits = kTightMaxBits;
         tcheck = true;
@@ -560,11 +573,11 @@ __global__ void __launch_bounds__(NT) stage_kernel(const StageArgs a) {
 
     // pass 3: magnitude of w*(y - c)
     double vmax = 0.0;
-    for (long long i = threadIdx.x; i < n; i += (int)blockDim.x) {
+    for (long long i = threadIdx.x; i < n; i += NT) {
         const double wi = w ? (double)w[i] : 1.0;
         vmax = max(vmax, fabs(wi * ((double)y[i] - shift)));
     }
-    vmax = block_max_d(vmax, shd);
+    vmax = block_max_d<NT>(vmax, shd);
     const int s_y = q_scale(vmax, qbits_y);
 
     // pass 4: staged arrays (padded with zero-weight points) and totals.
@@ -592,7 +605,7 @@ __global__ void __launch_bounds__(NT) stage_kernel(const StageArgs a) {
     const bool ilv = n > 1 && width > 0.0 && tmax >= width * (double)(n - 1);
     const long long n_full = ilv ? n_pad / kChunk * kChunk : 0;
     long long qw_tot = 0, qy_tot = 0, qy_abs = 0;
-    for (long long i = threadIdx.x; i < n_pad; i += (int)blockDim.x) {
+    for (long long i = threadIdx.x; i < n_pad; i += NT) {
         double d = 0.0;
         int qa = 0, qb = 0;
         if (i < n) {
@@ -616,9 +629,9 @@ __global__ void __launch_bounds__(NT) stage_kernel(const StageArgs a) {
         qy_tot += qb;
         qy_abs += qb < 0 ? -(long long)qb : (long long)qb;
     }
-    qw_tot = block_sum_ll(qw_tot, shl);
-    qy_tot = block_sum_ll(qy_tot, shl);
-    qy_abs = block_sum_ll(qy_abs, shl);
+    qw_tot = block_sum_ll<NT>(qw_tot, shl);
+    qy_tot = block_sum_ll<NT>(qy_tot, shl);
+    qy_abs = block_sum_ll<NT>(qy_abs, shl);
 
     if (threadIdx.x == 0) {
         const int nd = a.dur_cnt[c];
@@ -2391,14 +2404,16 @@ bool plan_shape(const atb_params* prm, int* nt, int* minb) {
     return false;
 }
 
-// Threads per stage CTA.  A batch of more points than n_sm curves of its longest
-// length is bound by throughput, and the smallest CTAs waste least (300 curves of
-// 1000 / 15 000 points: 26 / 151 us with 256 threads, 43 / 154 with 512, 89 / 191 with
-// 1024).  In others the longest curve's CTA is the last: 512 threads up to kStageLong
-// points (one curve of 4000 / 15 000 points: 34 / 59 us against 39 / 74 with 256 and 42 / 62
-// with 1024), 1024 beyond (40 000 points: 137 us against 147 with 512 and 216 with 256).
+// Threads per stage CTA.  A batch of more points than n_sm curves of its longest length
+// is bound by throughput: 256 threads waste least on short curves (300 curves of 1000 / 4000
+// points: 24 / 50 us against 38 / 55 with 512 and 80 / 95 with 1024), 512 are best beyond
+// (300 of 15 000 / 40 000: 139 / 406, 123 / 367, 170 / 412 us; 2000 of 15 000: 600, 503,
+// 764).  In others the longest curve's CTA is the last: 512 threads up to kStageLong points
+// (one curve of 4000 / 15 000 points: 28 / 49 us against 32 / 65 with 256 and 37 / 55 with
+// 1024), 1024 beyond (100 of 40 000 points: 141 us against 157 with 512 and 256 with 256).
 int stage_threads(int n_sm, long long n_longest, long long n_all) {
-    if (n_all > n_sm * n_longest) return kStageBlockS;
+    if (n_all > n_sm * n_longest)
+        return n_longest < kStageShort ? kStageBlockS : kStageBlockM;
     return n_longest < kStageLong ? kStageBlockM : kStageBlock;
 }
 
