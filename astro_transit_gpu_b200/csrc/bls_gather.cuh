@@ -63,6 +63,10 @@ constexpr long long kGatherMinPeriods = 32;      // of a curve
 // point, while the rest of the GPU waits for it, and by up to 600 CTAs at a time.
 constexpr long long kTableLatency = 12000;       // per point of the longest curve
 constexpr long long kTablePrice = kTableLatency / 600;  // per point of every curve
+// And what no sum over periods shows, about 40 us: the kernels of the look-up search itself and
+// its last, half-empty wave (of 133 batches of 12 000 to 250 000 periods that took the
+// tables, ten took longer for it, by 18 to 160 us; with this four).
+constexpr double kGatherPrice = 4.65e7;
 constexpr int kPriceClasses = 24;                // curve lengths by quarters of an octave
 constexpr int kHeadMax = 17;                     // saved prefix entries 0..oversample (<= 16)
 
@@ -151,18 +155,23 @@ struct GatherArgs {
 //     scan, windows) and 2.6 per point of the last bin where max_bins cuts the period (they
 //     add to one address); gathering 0.39 per look-up -- whole blocks of 128 per cycle -- and
 //     2.2 per bin; within 20 % of the times.  Weighted: 0.37, 3.7, 3.3; 0.75, 1.9 and
-//     a few hundred per period.
+//     a few hundred per period.  Of the bins' share, windows of one duration cost gathering
+//     0.10 clocks less (0.20 weighted): 64 weighted curves of 20 000 points, 2000 periods of
+//     678 bins on average gain 7 % with six durations, nothing with two and 20 % with twenty.
 //   fixed bins, whose look-ups take a cache line each: 0.8 to 1.5 per look-up (weighted
 //     2 to 3.3).  One look-up for five points (weighted: ten) breaks even: 15 000 points,
 //     200 bins and 10 cycles scatter in 5500 clocks and gather in 4400; 150 000 points, 300
 //     bins and 40 cycles in 43 000 and 31 000, 119 cycles in 38 500 and 71 400.
+//     Neighbouring periods share lines unless the grid is so coarse (`step`) that their
+//     boundaries lie far apart: 160 curves of 15 286 points, 333 bins, took 774 us scattered
+//     and 939 gathered by 209 periods from 1.5 to 23 d.
 //     Where the prefix entries leave an SM one CTA (from 320 bins, `one_cta`), a period
 //     costs 5 clocks per bin more (weighted 2.5): 500 bins and one cycle of 15 000 points
 //     scatter in 7800 clocks and gather in 8100.
 template <int GEOM>
 __device__ __forceinline__ double gather_gain(const CurveStat& st, int n, int lmax, double P,
-                                              int NB, int os, int cap, bool one_cta,
-                                              double& look) {
+                                              double step, int NB, int os, int cap,
+                                              bool one_cta, double& look) {
     // (a period beyond 64 spans would leave the table's number range)
     if (!(P > 0.0) || !(P <= 64.0 * st.dt_absmax)) return -INFINITY;
     const double cycles = floor(st.dt_absmax * (1.0 / P)) + 1.0;
@@ -174,12 +183,15 @@ __device__ __forceinline__ double gather_gain(const CurveStat& st, int n, int lm
         // once per bin-range pass
         const double passes =
             NB + 2 > cap ? ceil((double)NB / (double)max(cap - 2 - lmax, 64)) : 1.0;
+        const double nd = (double)st.n_dur;
         const double cut = fmax(0.0, 1.0 - (double)NB / (P * st.inv_bin_dur));
         look = (cnt ? 1.54 : 3.0) * cycles * 128.0 * ceil(bounds * (1.0 / 128.0));
         return (double)n * ((cnt ? 0.92 : 1.49) * passes + (cnt ? 10.4 : 13.3) * cut) +
-               (cnt ? 5.2 : 7.3) * bounds - look - (cnt ? 0.0 : 1500.0);
+               (cnt ? 2.3 + 0.41 * nd : 1.4 + 0.8 * nd) * bounds - look - (cnt ? 0.0 : 1500.0);
     }
-    look = (cnt ? 5.0 : 10.0) * cycles * 128.0 * ceil(((double)NB + 1.0) * (1.0 / 128.0));
+    const double apart = step * cycles * 0.5 * (double)n / st.dt_absmax;  // cells
+    look = (cnt ? 5.0 : 10.0) * cycles * 128.0 * ceil(((double)NB + 1.0) * (1.0 / 128.0)) *
+           (1.0 + 0.6 * fmin(1.0, apart * (1.0 / 96.0)));
     return (double)n - look - (one_cta ? (cnt ? 20.0 : 10.0) * (double)NB : 0.0);
 }
 
@@ -415,7 +427,8 @@ __global__ void __launch_bounds__(kTableBlock) gain_kernel(const SearchArgs a, c
                                : a.n_bins_fixed;
             double look = 0.0;
             const double gain = gather_gain<GEOM>(
-                sg, (int)n, lmax, P, NB, a.oversample, a.cap, one_cta, look);
+                sg, (int)n, lmax, P, fabs(a.periods[a.per_beg[c] + (i + 1 < np ? i + 1 : i - 1)] - P),
+                NB, a.oversample, a.cap, one_cta, look);
             // astropy bins: every period that can be, or none -- the look-ups per point
             // hardly depend on the period, and a curve split over both kernels took
             // longer than in either; fixed bins: the periods that gain
@@ -472,7 +485,7 @@ __device__ __forceinline__ int priced_class(const GatherPrice& p, int warps) {
         const double idle = fmax(0.0, (double)warps / (double)periods - 1.0);
         const double net = (double)saved - (double)looks * idle -
                            fmax((double)kTableLatency * (double)p.longest[k],
-                                (double)kTablePrice * (double)points);
+                                (double)kTablePrice * (double)points) - kGatherPrice;
         if (net >= best) {
             best = net;
             last = k;
