@@ -1847,12 +1847,23 @@ __device__ void run_group(const SearchArgs& a, GroupSmem& gs, longlong2* H, cons
     }
 }
 
+// First statement of the search's kernels, which are launched as a chain (launch_search):
+// the next kernel's CTAs may take their places once all of this one's have, and this one's
+// go on when the kernel before has ended and its writes are seen.  Nothing is read
+// or written before that, and no CTA ends before it, so that the end of one kernel
+// implies the end of all before it.
+__device__ __forceinline__ void chain_start() {
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
 #include "bls_gather.cuh"
 
 template <int GEOM, int NT, int MINB>
 __global__ void __launch_bounds__(NT, MINB) search_kernel(const SearchArgs a) {
     extern __shared__ __align__(16) longlong2 s_hist[];
     __shared__ GroupSmem gs;
+    chain_start();
     if (a.n_scatter && *a.n_scatter == 0) return;
 
     for (;;) {
@@ -2438,24 +2449,44 @@ GatherFn gather_fn(int geom, bool packed) {
     return packed ? gather_kernel<ATB_GEOM_FIXED, true> : gather_kernel<ATB_GEOM_FIXED, false>;
 }
 
-// The search: gathered periods (when the plan has tables), then scattered ones.
+// Launches a kernel of the search's chain, see chain_start.
+template <typename... P, typename... A>
+cudaError_t launch_chained(void (*fn)(P...), int grid, int block, int smem, cudaStream_t s,
+                           A&&... args) {
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3((unsigned)grid);
+    cfg.blockDim = dim3((unsigned)block);
+    cfg.dynamicSmemBytes = (size_t)smem;
+    cfg.stream = s;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, fn, std::forward<A>(args)...);
+}
+
+// The search: gathered periods (when the plan has tables), then scattered ones.  The
+// kernels of a plan with tables are chained: where none is made they end at once, one
+// after another, and their launches cost more than they do (82 curves of 4915 points, 312
+// periods, 183 bins: 241 us without tables, 257 launched one by one; 235 and 242 chained).
 int launch_search(atb_plan* p, cudaStream_t s) {
-    if (p->ga.tab) {
-        const bool binned = p->prm.geometry == ATB_GEOM_BINNED;
-        (binned ? gain_kernel<ATB_GEOM_BINNED> : gain_kernel<ATB_GEOM_FIXED>)
-            <<<p->n_curves, kTableBlock, 0, s>>>(p->qa, p->ga, p->tstats);
+    const SearchFn search = search_fn(p->prm.geometry, p->nt);
+    if (!p->ga.tab) {
+        search<<<p->grid, p->nt, p->smem_bytes, s>>>(p->qa);
         ATB_CUDA(p->h, cudaGetLastError());
-        (binned ? table_kernel<ATB_GEOM_BINNED> : table_kernel<ATB_GEOM_FIXED>)
-            <<<p->n_curves, kTableBlock, 0, s>>>(p->qa, p->ga, p->tstats);
-        ATB_CUDA(p->h, cudaGetLastError());
-        for (int w = 0; w < p->ga.vs; ++w) {  // counting curves, then weighted ones
-            gather_fn(p->prm.geometry, w == 0)<<<p->gather_grid[w], kGatherBlock, p->gather_smem[w],
-                                                 s>>>(p->qa, p->ga);
-            ATB_CUDA(p->h, cudaGetLastError());
-        }
+        return ATB_OK;
     }
-    search_fn(p->prm.geometry, p->nt)<<<p->grid, p->nt, p->smem_bytes, s>>>(p->qa);
-    ATB_CUDA(p->h, cudaGetLastError());
+    const bool binned = p->prm.geometry == ATB_GEOM_BINNED;
+    ATB_CUDA(p->h, launch_chained(binned ? gain_kernel<ATB_GEOM_BINNED> : gain_kernel<ATB_GEOM_FIXED>,
+                                  p->n_curves, kTableBlock, 0, s, p->qa, p->ga, p->tstats));
+    ATB_CUDA(p->h,
+             launch_chained(binned ? table_kernel<ATB_GEOM_BINNED> : table_kernel<ATB_GEOM_FIXED>,
+                            p->n_curves, kTableBlock, 0, s, p->qa, p->ga, p->tstats));
+    for (int w = 0; w < p->ga.vs; ++w)  // counting curves, then weighted ones
+        ATB_CUDA(p->h, launch_chained(gather_fn(p->prm.geometry, w == 0), p->gather_grid[w],
+                                      kGatherBlock, p->gather_smem[w], s, p->qa, p->ga));
+    ATB_CUDA(p->h, launch_chained(search, p->grid, p->nt, p->smem_bytes, s, p->qa));
     return ATB_OK;
 }
 

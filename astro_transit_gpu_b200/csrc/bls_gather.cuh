@@ -390,6 +390,7 @@ template <int GEOM>
 __global__ void __launch_bounds__(kTableBlock) gain_kernel(const SearchArgs a, const GatherArgs ga,
                                                            TableStat* stats) {
     __shared__ TableShared sh;
+    chain_start();
     const int c = blockIdx.x, tid = threadIdx.x;
     const long long n = a.pt_off[c + 1] - a.pt_off[c];
     const long long cells = ga.cell_off[c + 1] - ga.cell_off[c];
@@ -499,6 +500,7 @@ template <int GEOM>
 __global__ void __launch_bounds__(kTableBlock) table_kernel(const SearchArgs a, const GatherArgs ga,
                                                             TableStat* stats) {
     __shared__ TableShared sh;
+    chain_start();
     const int c = blockIdx.x, tid = threadIdx.x;
     if (!stats[c].g_on) return;
     TableStat sg = stats[c];
@@ -1660,6 +1662,7 @@ __global__ void __launch_bounds__(kGatherBlock, kGatherMinBlocks)
     extern __shared__ __align__(16) char g_smem[];
     __shared__ long long s_beg, s_end;  // the part's periods (s_beg < 0: no more parts)
     __shared__ int s_curve;
+    chain_start();
     if (ga.n_gather[PK ? 0 : 1] == 0) return;
     const int warp = threadIdx.x >> 5;
     const unsigned fsz = gather_ring_bytes(ga.ring);
