@@ -723,7 +723,7 @@ constexpr int kMaxList = 64;  // windows within reach of the best, before the ex
 struct FilterState {
     float lim;
     float eA;      // astropy bins: e0; fixed bins: the whole error bound E of the period
-    float wE, wN, wm;  // GatherConsts
+    float wE, wN;  // GatherConsts
 };
 
 // Shared memory of one warp besides its prefix entries.
@@ -741,6 +741,7 @@ struct WarpState {
     Sum<PK> A0, tot;             // sum before boundary 0; totals
     Sum<PK> cm1, hnb;            // astropy bins: C[M-1] and C[NB] - C[NB-1] of the padding copy
     FilterState f;
+    float wm;                    // GatherConsts; weighted curves only
     float guess;                 // see gather_period
     const TableStat* st;
     const Entry<PK>* tab;
@@ -1149,6 +1150,8 @@ __device__ __noinline__ float gather_pass(WarpState<PK>* ws, unsigned base, unsi
                                           bool ok, int k0, int k1) {
     const int lane = threadIdx.x & 31;
     FilterState f = ws->f;
+    float wm = 0.0f;
+    if constexpr (!PK) wm = ws->wm;
     const int nd = ws->st->n_dur;
     const float up = 1.0f + 3.814697265625e-06f, dn = 1.0f - 3.814697265625e-06f;  // 2^-18
     const unsigned as = base + 8u * (unsigned)s;
@@ -1168,9 +1171,11 @@ __device__ __noinline__ float gather_pass(WarpState<PK>* ws, unsigned base, unsi
         const float den0 = dw * (f.wN - dw);
         // weighted: a window holds a point, or is none; with fixed bins, whose windows
         // count no point twice, so does the rest of the curve
-        const float di = PK ? dw : fmaxf(dw, f.wm);
-        const float wo = PK || GEOM == ATB_GEOM_BINNED ? f.wN - di : fmaxf(f.wN - di, f.wm);
-        const float den = PK ? den0 : di * wo;
+        float den = den0;
+        if constexpr (!PK) {
+            const float di = fmaxf(dw, wm);
+            den = di * (GEOM == ATB_GEOM_BINNED ? f.wN - di : fmaxf(f.wN - di, wm));
+        }
         const float num = GEOM == ATB_GEOM_BINNED ? t * fabsf(t) : t * t;
         // An entry beyond the last is NaN: no window.  No weight inside or outside is
         // none either (the padding copy can put more than the total inside).
@@ -1229,13 +1234,16 @@ __device__ __noinline__ void gather_windows(WarpState<PK>* ws, unsigned base, un
                                             int nd, int k0, int s_beg, int s_end) {
     const int lane = threadIdx.x & 31;
     FilterState f = ws->f;
+    float wm = 0.0f;
+    if constexpr (!PK) wm = ws->wm;
     unsigned l8[KC];
 #pragma unroll
     for (int q = 0; q < KC; ++q) l8[q] = 8u * (unsigned)min(ws->len[min(k0 + q, nd - 1)], 1 << 24);
     for (int s0 = s_beg; s0 < s_end; s0 += 64) {
         // (1 - 2^-20): the rounding of lim * wN - lim * dw stays on the safe side
         const float lN = -f.lim * f.wN * 0.99999904632568359375f;
-        const float lm = -f.lim * f.wm * 0.99999904632568359375f;
+        float lm = 0.0f;
+        if constexpr (!PK) lm = -f.lim * wm * 0.99999904632568359375f;
         float top[2];
 #pragma unroll
         for (int i = 0; i < 2; ++i) {
@@ -1249,7 +1257,8 @@ __device__ __noinline__ void gather_windows(WarpState<PK>* ws, unsigned base, un
             for (int q = 0; q < KC; ++q) {
                 const float2 v = ent_add(min(as + l8[q], last), n);
                 const float t = GEOM == ATB_GEOM_BINNED ? v.x : fabsf(v.x) + f.eA;
-                const float dw = PK ? v.y : fmaxf(v.y, f.wm);
+                float dw = v.y;
+                if constexpr (!PK) dw = fmaxf(dw, wm);
                 float a = fmaf(f.lim, dw, lN);
                 if (!PK && GEOM == ATB_GEOM_FIXED) a = fminf(a, lm);
                 const float r = fmaf(a, dw, GEOM == ATB_GEOM_BINNED ? t * fabsf(t) : t * t);
@@ -1470,7 +1479,8 @@ __device__ __forceinline__ bool gather_period(const SearchArgs& a, WarpState<PK>
         if (lane == 0) {
             const GatherConsts& gk = ws.st->gk;
             ws.n_list = 0;
-            ws.f = FilterState{guess, gk.e0, gk.wE, gk.wN, gk.wm};
+            ws.f = FilterState{guess, gk.e0, gk.wE, gk.wN};
+            if constexpr (!PK) ws.wm = gk.wm;
             ws.tot = curve_total<PK>(*ws.st);
         }
         __syncwarp();
