@@ -772,7 +772,7 @@ struct GroupSmem {
     int key[kMaxWarps];
     long long tile;
     long long pb;
-    unsigned long long todo;  // the tile's periods still to search: one bit each
+    unsigned todo[2];         // the tile's periods still to search: one bit each
     int np;                   // the tile's periods, those of the gather kernel included
     int next;                 // first period after the group
     int curve;
@@ -1898,32 +1898,28 @@ __global__ void __launch_bounds__(NT, MINB) search_kernel(const SearchArgs a) {
             gs.dur[threadIdx.x] = a.durations[a.dur_beg[c] + threadIdx.x];
         }
         // the tile's periods and bin counts, loaded in parallel, and a bit for each
-        // that is not the gather kernel's: two ballots by the first warp
+        // that is not the gather kernel's: a ballot by each of the first two warps
         const long long p0 = gs.pb;
-        const int np = gs.np;
-        static_assert(kTileP <= 64 && NT >= kTileP, "one bit and one thread per period");
-        if (threadIdx.x < 32) {
-            const unsigned char* sc = a.scatter ? a.scatter + a.flag_off[c] + p0 : nullptr;
+        static_assert(kTileP == 64 && NT >= kTileP, "one bit and one thread per period");
+        if (threadIdx.x < kTileP) {
             const int i = threadIdx.x;
-            const unsigned lo = __ballot_sync(0xffffffffu, i < np && (!sc || sc[i]));
-            const unsigned hi = __ballot_sync(0xffffffffu, 32 + i < np && (!sc || sc[32 + i]));
-            if (i == 0) gs.todo = (unsigned long long)hi << 32 | lo;
-        }
-        __syncthreads();
-        const unsigned long long todo = gs.todo;
-        if (threadIdx.x < kTileP && (todo >> threadIdx.x & 1ULL)) {
-            const int i = threadIdx.x;
-            double P = a.periods[pbeg + p0 + i];
-            if (!(P > 0.0) || !(P < 1.0e300)) {
+            double P = i < gs.np ? a.periods[pbeg + p0 + i] : 1.0;
+            const bool mine = i < gs.np && (!a.scatter || a.scatter[a.flag_off[c] + p0 + i] != 0);
+            const unsigned who = __ballot_sync(0xffffffffu, mine);
+            if (i % 32 == 0) gs.todo[i / 32] = who;
+            if (mine && (!(P > 0.0) || !(P < 1.0e300))) {
                 atomicOr(a.status, 4);
                 P = 1.0;
             }
-            gs.tP[i] = P;
-            gs.tNB[i] = (GEOM == ATB_GEOM_BINNED)
-                            ? binned_nbins(P, st.inv_bin_dur, a.oversample, a.max_bins)
-                            : a.n_bins_fixed;
+            if (mine) {
+                gs.tP[i] = P;
+                gs.tNB[i] = (GEOM == ATB_GEOM_BINNED)
+                                ? binned_nbins(P, st.inv_bin_dur, a.oversample, a.max_bins)
+                                : a.n_bins_fixed;
+            }
         }
         __syncthreads();
+        const unsigned long long todo = (unsigned long long)gs.todo[1] << 32 | gs.todo[0];
         int pn = todo ? __ffsll((long long)todo) - 1 : kTileP;
         while (pn < kTileP) {
             if (threadIdx.x == 0) {
