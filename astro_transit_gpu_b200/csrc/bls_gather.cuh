@@ -64,8 +64,9 @@ constexpr long long kGatherMinPeriods = 32;      // of a curve
 constexpr long long kTableLatency = 12000;       // per point of the longest curve
 constexpr long long kTablePrice = kTableLatency / 600;  // per point of every curve
 // And what no sum over periods shows, about 40 us: the kernels of the look-up search itself and
-// its last, half-empty wave (of 133 batches of 12 000 to 250 000 periods that took the
-// tables, ten took longer for it, by 18 to 160 us; with this four).
+// its last, half-empty wave.  (500 drawn batches of 12 000 to 250 000 periods: 133 took the
+// tables without it, ten of them longer for it, by up to 160 us; with it, and with the
+// shares of gather_gain as they are now, 122 and five, by up to 60.)
 constexpr double kGatherPrice = 4.65e7;
 constexpr int kPriceClasses = 24;                // curve lengths by quarters of an octave
 constexpr int kHeadMax = 17;                     // saved prefix entries 0..oversample (<= 16)
@@ -153,10 +154,10 @@ struct GatherArgs {
 // of 0.6 to 150 d, 6 and 8 durations, 0.002 and 0.004 d bins; 592 periods of 32 curves):
 //   astropy bins, counting: scattering 0.23 clocks per point and pass, 3.5 per bin (clear,
 //     scan, windows) and 2.6 per point of the last bin where max_bins cuts the period (they
-//     add to one address); gathering 0.39 per look-up -- whole blocks of 128 per cycle -- and
-//     2.2 per bin; within 20 % of the times.  Weighted: 0.37, 3.7, 3.3; 0.75, 1.9 and
-//     a few hundred per period.  Of the bins' share, windows of one duration cost gathering
-//     0.10 clocks less (0.20 weighted): 64 weighted curves of 20 000 points, 2000 periods of
+//     add to one address); gathering 0.34 per look-up -- whole blocks of 128 per cycle -- and
+//     2.2 per bin; within 20 % of the times.  Weighted: 0.37, 3.7, 3.3; 0.71, 1.9 and
+//     500 per period.  Of the bins' share, windows of one duration cost gathering
+//     0.10 clocks less (0.25 weighted): 64 weighted curves of 20 000 points, 2000 periods of
 //     678 bins on average gain 7 % with six durations, nothing with two and 20 % with twenty.
 //   fixed bins, whose look-ups take a cache line each: 0.8 to 1.5 per look-up (weighted
 //     2 to 3.3).  One look-up for five points (weighted: ten) breaks even: 15 000 points,
@@ -185,9 +186,9 @@ __device__ __forceinline__ double gather_gain(const CurveStat& st, int n, int lm
             NB + 2 > cap ? ceil((double)NB / (double)max(cap - 2 - lmax, 64)) : 1.0;
         const double nd = (double)st.n_dur;
         const double cut = fmax(0.0, 1.0 - (double)NB / (P * st.inv_bin_dur));
-        look = (cnt ? 1.54 : 3.0) * cycles * 128.0 * ceil(bounds * (1.0 / 128.0));
+        look = (cnt ? 1.35 : 2.85) * cycles * 128.0 * ceil(bounds * (1.0 / 128.0));
         return (double)n * ((cnt ? 0.92 : 1.49) * passes + (cnt ? 10.4 : 13.3) * cut) +
-               (cnt ? 2.3 + 0.41 * nd : 1.4 + 0.8 * nd) * bounds - look - (cnt ? 0.0 : 1500.0);
+               (cnt ? 2.3 + 0.41 * nd : 0.2 + nd) * bounds - look - (cnt ? 0.0 : 2000.0);
     }
     const double apart = step * cycles * 0.5 * (double)n / st.dt_absmax;  // cells
     look = (cnt ? 5.0 : 10.0) * cycles * 128.0 * ceil(((double)NB + 1.0) * (1.0 / 128.0)) *
@@ -414,13 +415,14 @@ __global__ void __launch_bounds__(kTableBlock) gain_kernel(const SearchArgs a, c
              a.oversample < kHeadMax && lmax <= ga.ring - 192 &&
              // (a period's look-ups are at least T / b, and bin-range passes rarely double
              // the scattering)
-             T * sg.inv_bin_dur <= 1.36 * (double)n;
+             T * sg.inv_bin_dur <= 1.55 * (double)n;
     else
         on = on && 2 * a.n_bins_fixed + 1 <= ga.ring;
     unsigned char* scatter = a.scatter + a.flag_off[c];
     long long n_g = 0, saved = 0, looks = 0;
     if (on) {
         const bool one_cta = ga.one_cta[sg.cnt_win ? 0 : 1] != 0;
+#pragma unroll 4
         for (long long i = tid; i < np; i += kTableBlock) {
             const double P = a.periods[a.per_beg[c] + i];
             const int NB = GEOM == ATB_GEOM_BINNED
