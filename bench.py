@@ -233,6 +233,10 @@ def curve_periods(periods, c):
     return periods[c] if isinstance(periods, list) else periods
 
 
+def curve_durations(durations, c):
+    return durations[c] if np.ndim(durations[0]) else durations
+
+
 def flat(a):
     return np.concatenate(a) if isinstance(a, list) else a
 
@@ -646,7 +650,7 @@ def main(argv=None):
     g = plan.gathered()  # of the last profiled execution
     n_per = sum(len(curve_periods(periods, c)) for c in range(nc))
     gathered = (g["counting"] + g["weighted"] - g["given_back"]) / max(n_per, 1)
-    lookups = (sum(table_lookups(t[c], curve_periods(periods, c), curve_periods(durs, c))
+    lookups = (sum(table_lookups(t[c], curve_periods(periods, c), curve_durations(durs, c))
                    for c in range(nc)) if gathered == 1.0 and args.method == "parity" else None)
     layout_share = {LAYOUT_NAMES[k]: float(upd[layout == k].sum() / u_fold)
                     for k in LAYOUT_NAMES}

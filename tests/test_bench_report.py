@@ -38,3 +38,8 @@ def test_table_lookups():
     t = np.linspace(0.0, 10.0, 1000)
     got = bench.table_lookups(t, np.array([2.5, 12.0]), np.array([0.04, 0.08]))
     assert got == 5 * 5 * 128 + 24 * 128
+
+
+def test_durations_shared_or_per_curve():
+    assert bench.curve_durations([0.04, 0.08], 5) == [0.04, 0.08]
+    assert bench.curve_durations([np.array([0.04]), np.array([0.08])], 1)[0] == 0.08
