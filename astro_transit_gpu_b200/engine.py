@@ -497,7 +497,9 @@ class BLSEngine:
             key = torch.zeros(nc, dtype=torch.int64, device=batch.device)
             best = torch.empty(nc, dtype=torch.int32, device=batch.device)
         # (stream-ordered: a plan of device-wide allocations maps and unmaps its memory
-        # on every call, and waits for other streams' work)
+        # on every call, and waits for other streams' work; the caller's, which may still
+        # be writing the batch, is waited for)
+        s.wait_stream(torch.cuda.current_stream(batch.device))
         plan = self.plan(batch, config, {"best_key": key, "best_period": best}, stream=s)
         try:
             plan.execute(s)

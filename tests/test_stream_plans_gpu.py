@@ -56,3 +56,23 @@ def test_screen(streams_of_plans):
     assert None not in streams_of_plans
     assert np.array_equal(got["best_index"].cpu().numpy(), full.argmax(1))
     assert np.array_equal(got["power"].cpu().numpy(), full.max(1))
+
+
+def test_screen_waits_for_the_callers_stream():
+    """The batch may still be on its way when screen is called with another stream."""
+    import torch
+    from astro_transit_gpu_b200.engine import BLSEngine, CurveBatch, SearchConfig
+    t, y = _curves()
+    batch = CurveBatch.from_arrays(t, y, periods=np.linspace(0.6, 4.0, 400),
+                                   durations=np.array([0.05, 0.1]))
+    engine, cfg = BLSEngine.get(), SearchConfig("fast", n_bins=200)
+    want = engine.screen(batch, cfg)
+    flux = batch.y.clone()
+    batch.y.copy_(torch.flip(flux, (0,)))
+    s = torch.cuda.Stream()
+    torch.cuda.synchronize()
+    torch.cuda._sleep(100_000_000)  # about 50 ms of the caller's stream
+    batch.y.copy_(flux)
+    got = engine.screen(batch, cfg, stream=s)
+    for k, v in want.items():
+        assert torch.equal(got[k], v), k
