@@ -2263,7 +2263,7 @@ struct atb_plan {
     };
     Control* control = nullptr;
     int* status = nullptr;
-    // prefix-gather search (its tables exist when ga.off is set)
+    // prefix-gather search (its tables exist when ga.tab is set)
     GatherArgs ga{};
     TableStat* tstats = nullptr;
     int gather_grid[2] = {0, 0};  // packed, weighted

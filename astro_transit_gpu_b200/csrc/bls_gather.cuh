@@ -30,10 +30,11 @@
 // change their width with the period; their cells are stored in order.
 //
 // One warp searches one period: it gathers 128 boundaries at a time into a buffer of
-// 384 FP32 prefix entries (3 KB) and evaluates the windows that end inside it, so
-// a period of any number of bins needs no more, and no barrier.  Bound by issue slots
-// and look-up latency: 128 curves of 15 000 points, 5000 periods and 0.004 d bins take
-// 11.7 ms against 14.35 ms scattered.
+// FP32 prefix entries and evaluates the windows that end inside it.  With astropy bins
+// the buffer slides, so 384 entries (3 KB) do for a period of any number of bins; fixed
+// bins hold the period twice (up to kMaxRing entries).  The warps of a CTA wait for one
+// another after each period only to share table lines and instructions
+// (gather_periods).  Bound by issue slots and look-up latency.
 
 // 16 warps share table lines and instructions; 8 took 2.15 ms where 16 took 1.95
 // (16 one-sector curves), 32 were slower on full batches
@@ -126,7 +127,7 @@ struct TableStat : CurveStat {
     int g_pitch;     // entries per row
     int g_colmax;    // last column a look-up may use
     int lmax;        // longest window in bins (astropy bins)
-    double g_scale;  // table units (2^-20 cell) per unit time
+    double g_scale;  // table units (2^-24 cell) per unit time
     long long n_g;   // periods that are gathered
     GatherConsts gk;
 };
@@ -1229,8 +1230,8 @@ __device__ __noinline__ float gather_pass(WarpState<PK>* ws, unsigned base, unsi
 // with t an upper bound of sigma, evaluated as two fused multiply-adds (weighted:
 // dw no less than wm, see GatherConsts).  The entry
 // at `last`, where longer windows end, is NaN, and r is too.
-// (Out of line, one instance per KC: copies of this loop specialised by caller
-// and range made the kernel miss the instruction cache.)
+// (Out of line, KC = 3 for every call: copies of this loop specialised by caller,
+// number of lengths and range made the kernel miss the instruction cache.)
 template <int GEOM, bool PK, int KC>
 __device__ __noinline__ void gather_windows(WarpState<PK>* ws, unsigned base, unsigned last,
                                             int nd, int k0, int s_beg, int s_end) {
