@@ -1848,13 +1848,18 @@ __device__ void run_group(const SearchArgs& a, GroupSmem& gs, longlong2* H, cons
 }
 
 // First statement of the search's kernels, which are launched as a chain (launch_search):
-// the next kernel's CTAs may take their places once all of this one's have, and this one's
-// go on when the kernel before has ended and its writes are seen.  Nothing is read
-// or written before that, and no CTA ends before it, so that the end of one kernel
-// implies the end of all before it.
+// the next kernel is started as soon as this one's CTAs have ended or called chain_next, and
+// its CTAs go on when all of this one's have ended and their writes are seen.  Nothing is
+// read or written before that, and no CTA ends before it, so that the end of one kernel
+// implies the end of all before it.  Only gain_kernel, a few microseconds long, calls
+// chain_next: CTAs that wait hold their places, which the plans of other streams could use
+// (85 curves of 34 536 points, 1974 periods, as a session of four streams: 4.72 ms when
+// every kernel called it, 4.31 so).
 __device__ __forceinline__ void chain_start() {
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+__device__ __forceinline__ void chain_next() {
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 
 #include "bls_gather.cuh"
@@ -2465,7 +2470,7 @@ cudaError_t launch_chained(void (*fn)(P...), int grid, int block, int smem, cuda
 // The search: gathered periods (when the plan has tables), then scattered ones.  The
 // kernels of a plan with tables are chained: where none is made they end at once, one
 // after another, and their launches cost more than they do (82 curves of 4915 points, 312
-// periods, 183 bins: 241 us without tables, 257 launched one by one; 235 and 242 chained).
+// periods, 183 bins: 241 us without tables, 257 launched one by one; 254 and 262 chained).
 int launch_search(atb_plan* p, cudaStream_t s) {
     const SearchFn search = search_fn(p->prm.geometry, p->nt);
     if (!p->ga.tab) {

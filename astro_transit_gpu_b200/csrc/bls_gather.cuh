@@ -392,6 +392,7 @@ template <int GEOM>
 __global__ void __launch_bounds__(kTableBlock) gain_kernel(const SearchArgs a, const GatherArgs ga,
                                                            TableStat* stats) {
     __shared__ TableShared sh;
+    chain_next();
     chain_start();
     const int c = blockIdx.x, tid = threadIdx.x;
     const long long n = a.pt_off[c + 1] - a.pt_off[c];
