@@ -35,6 +35,7 @@ EXPORTS = (
     "atb_bench_smem_red_u64", "atb_bench_smem_red_u32", "atb_bench_dfma", "atb_search_curve_static",
     "atb_plan_curve_layout", "atb_plan_create_async", "atb_plan_top_k",
     "atb_plan_create_limited", "atb_plan_gathered", "atb_plan_table_bytes",
+    "atb_plan_create_beside",
 )
 
 # limit of atb_search_curve_static (ATB_STATIC_MAX_POINTS in the header)
@@ -102,6 +103,8 @@ def load(build_if_missing: bool = True):
         L.atb_plan_create_limited.argtypes = [_vp, ctypes.POINTER(Params), ctypes.POINTER(Batch),
                                               ctypes.POINTER(Outputs), _vp, _i64,
                                               ctypes.POINTER(_vp)]
+        L.atb_plan_create_beside.argtypes = [_vp, ctypes.POINTER(Params), ctypes.POINTER(Batch),
+                                             ctypes.POINTER(Outputs), _i32, ctypes.POINTER(_vp)]
         L.atb_plan_gathered.argtypes = [_vp, _i64p, _i64p, _i64p]
         L.atb_plan_execute.argtypes = [_vp, _vp]
         L.atb_plan_top_k.argtypes = [_vp, _i32, _i32, _vp, _vp]

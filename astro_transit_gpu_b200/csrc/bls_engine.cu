@@ -2511,10 +2511,11 @@ size_t free_bytes(const atb_plan* p) {
 // asks next (they take more than the curves themselves, 40 to 88 bytes per point, and the
 // batches of before they were made filled the device with less).
 int plan_gather(atb_plan* p, const std::vector<long long>& pt_off,
-                const std::vector<long long>& per_cnt, bool weighted, long long limit) {
+                const std::vector<long long>& per_cnt, bool weighted, long long limit, int beside) {
     if (limit == 0) return ATB_OK;
     const int nc = p->n_curves;
     GatherArgs ga{};
+    ga.beside = beside;
     ga.vs = weighted ? 2 : 1;
     ga.ring = 384;  // astropy bins: windows of up to 192 bins
     if (p->prm.geometry == ATB_GEOM_FIXED) {
@@ -2689,28 +2690,36 @@ int atb_last_error(const atb_handle* h, char* buf, size_t len) {
 
 namespace {
 int plan_create(atb_handle* h, const atb_params* prm, const atb_batch* b, const atb_outputs* o,
-                cudaStream_t stream, bool async, long long table_bytes, atb_plan** out);
+                cudaStream_t stream, bool async, long long table_bytes, int beside,
+                atb_plan** out);
 }  // namespace
 
 int atb_plan_create(atb_handle* h, const atb_params* prm, const atb_batch* b,
                     const atb_outputs* o, atb_plan** out) {
-    return plan_create(h, prm, b, o, nullptr, false, -1, out);
+    return plan_create(h, prm, b, o, nullptr, false, -1, 1, out);
+}
+
+int atb_plan_create_beside(atb_handle* h, const atb_params* prm, const atb_batch* b,
+                           const atb_outputs* o, int32_t beside, atb_plan** out) {
+    return plan_create(h, prm, b, o, nullptr, false, -1, std::min(std::max(beside, 1), 64), out);
 }
 
 int atb_plan_create_async(atb_handle* h, const atb_params* prm, const atb_batch* b,
                           const atb_outputs* o, void* stream, atb_plan** out) {
-    return plan_create(h, prm, b, o, static_cast<cudaStream_t>(stream), true, -1, out);
+    return plan_create(h, prm, b, o, static_cast<cudaStream_t>(stream), true, -1, 1, out);
 }
 
 int atb_plan_create_limited(atb_handle* h, const atb_params* prm, const atb_batch* b,
                             const atb_outputs* o, void* stream, int64_t table_bytes,
                             atb_plan** out) {
-    return plan_create(h, prm, b, o, static_cast<cudaStream_t>(stream), true, table_bytes, out);
+    return plan_create(h, prm, b, o, static_cast<cudaStream_t>(stream), true, table_bytes, 1,
+                       out);
 }
 
 namespace {
 int plan_create(atb_handle* h, const atb_params* prm, const atb_batch* b, const atb_outputs* o,
-                cudaStream_t stream, bool async, long long table_bytes, atb_plan** out) {
+                cudaStream_t stream, bool async, long long table_bytes, int beside,
+                atb_plan** out) {
     if (!h) return ATB_EINVAL;
     if (!prm || !b || !o || !out) return fail(h, ATB_EINVAL, "null argument");
     *out = nullptr;
@@ -2972,7 +2981,7 @@ int plan_create(atb_handle* h, const atb_params* prm, const atb_batch* b, const 
     qa.tile_counter = &p->control->tiles;
     qa.status = p->status;
     p->best = o->best_period;
-    if ((rc = plan_gather(p, pt_off, per_cnt, b->w != nullptr, table_bytes))) {
+    if ((rc = plan_gather(p, pt_off, per_cnt, b->w != nullptr, table_bytes, beside))) {
         plan_free(p);
         delete p;
         return rc;

@@ -147,6 +147,7 @@ struct GatherArgs {
     int one_cta[2];            // and whether they are one CTA per SM
     int vs;                    // 2 when weights are given, else 1
     int ring;                  // prefix entries a warp holds
+    int beside;                // plans that run at the same time, this one included
 };
 
 // What gathering a period saves, in quarters of an SM clock (about a scattered point of a
@@ -476,8 +477,10 @@ __global__ void __launch_bounds__(kTableBlock) gain_kernel(const SearchArgs a, c
 
 // The last class of lengths that gets tables (-1: none): with it, what they save less
 // what they cost is largest.  Too few periods leave warps of the gather kernel idle and
-// their look-ups take as much longer.
-__device__ __forceinline__ int priced_class(const GatherPrice& p, int warps) {
+// their look-ups take as much longer.  Of what only leaves the GPU idle, `beside` plans that
+// run at the same time each bear a share (24 curves of 34 536 points, 6000 periods, as a
+// session of four: 4.55 ms scattered, 3.36 by tables).
+__device__ __forceinline__ int priced_class(const GatherPrice& p, int warps, int beside) {
     long long saved = 0, looks = 0, periods = 0, points = 0;
     double best = 0.0;
     int last = -1;
@@ -487,10 +490,11 @@ __device__ __forceinline__ int priced_class(const GatherPrice& p, int warps) {
         looks += p.looks[k];
         periods += p.periods[k];
         points += p.points[k];
-        const double idle = fmax(0.0, (double)warps / (double)periods - 1.0);
+        const double idle = fmax(0.0, (double)(warps / beside) / (double)periods - 1.0);
         const double net = (double)saved - (double)looks * idle -
-                           fmax((double)kTableLatency * (double)p.longest[k],
-                                (double)kTablePrice * (double)points) - kGatherPrice;
+                           fmax((double)(kTableLatency / beside) * (double)p.longest[k],
+                                (double)kTablePrice * (double)points) -
+                           kGatherPrice / (double)beside;
         if (net >= best) {
             best = net;
             last = k;
@@ -516,7 +520,8 @@ __global__ void __launch_bounds__(kTableBlock) table_kernel(const SearchArgs a, 
     const long long n_full = st.ilv ? (n + kR - 1) / kR * kR / kChunk * kChunk : 0;
     const double* sdt = a.sdt + so;
     const double T = st.dt_absmax;
-    if (tid == 0) sh.flag = price_class(n) <= priced_class(*ga.price, ga.warps[st.cnt_win ? 0 : 1]);
+    if (tid == 0) sh.flag = price_class(n) <=
+                           priced_class(*ga.price, ga.warps[st.cnt_win ? 0 : 1], ga.beside);
     __syncthreads();
     bool on = sh.flag != 0;
     const long long most_shared = GEOM == ATB_GEOM_BINNED ? 0 : n / 512;

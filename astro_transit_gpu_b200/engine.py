@@ -204,10 +204,11 @@ class SearchPlan:
 
     def __init__(self, engine: "BLSEngine", batch: CurveBatch, config: SearchConfig,
                  outputs: Dict[str, torch.Tensor], stream: Optional[torch.cuda.Stream] = None,
-                 table_bytes: int = -1):
+                 table_bytes: int = -1, beside: int = 1):
         """With `stream`, the plan is set up and released in that stream's
         order (atb_plan_create_async) and must be executed on it; `table_bytes`
-        then limits its look-up tables (atb_plan_create_limited)."""
+        then limits its look-up tables (atb_plan_create_limited).  Without one,
+        `beside` plans are executed at the same time (atb_plan_create_beside)."""
         if stream is None and table_bytes >= 0:
             raise ValueError("table_bytes needs a stream")
         self.engine = engine
@@ -244,8 +245,9 @@ class SearchPlan:
         ptr = ctypes.c_void_p()
         with torch.cuda.device(batch.device):
             if stream is None:
-                rc = lib.atb_plan_create(engine.handle.ptr, ctypes.byref(self._params),
-                                         ctypes.byref(b), ctypes.byref(o), ctypes.byref(ptr))
+                rc = lib.atb_plan_create_beside(engine.handle.ptr, ctypes.byref(self._params),
+                                                ctypes.byref(b), ctypes.byref(o), int(beside),
+                                                ctypes.byref(ptr))
             else:
                 rc = lib.atb_plan_create_limited(engine.handle.ptr, ctypes.byref(self._params),
                                                  ctypes.byref(b), ctypes.byref(o),
@@ -475,11 +477,12 @@ class BLSEngine:
 
     def plan(self, batch: CurveBatch, config: SearchConfig,
              outputs: Optional[Dict[str, torch.Tensor]] = None,
-             stream: Optional[torch.cuda.Stream] = None, table_bytes: int = -1) -> SearchPlan:
+             stream: Optional[torch.cuda.Stream] = None, table_bytes: int = -1,
+             beside: int = 1) -> SearchPlan:
         if outputs is None:
             outputs = self.allocate_outputs(batch)
         return SearchPlan(self, batch, self.tuned_config(batch, config), outputs, stream,
-                          table_bytes)
+                          table_bytes, beside)
 
     def screen(self, batch: CurveBatch, config: SearchConfig,
                stream: Optional[torch.cuda.Stream] = None) -> Dict[str, torch.Tensor]:
@@ -583,7 +586,7 @@ class BatchSession:
 
     def __init__(self, engine: BLSEngine, point_offset: np.ndarray, periods, durations,
                  config: SearchConfig, y_dtype=np.float32, weighted: bool = True,
-                 fields: Sequence[str] = OUTPUT_FIELDS):
+                 fields: Sequence[str] = OUTPUT_FIELDS, beside: int = 1):
         dev = engine.device
         pt = _i64(point_offset)
         n_pts = int(pt[-1])
@@ -608,7 +611,7 @@ class BatchSession:
         self.outputs = BLSEngine.allocate_outputs(self.batch, fields)
         self.host_out = {k: torch.empty(v.shape, dtype=v.dtype).pin_memory()
                          for k, v in self.outputs.items()}
-        self.plan = engine.plan(self.batch, config, self.outputs)
+        self.plan = engine.plan(self.batch, config, self.outputs, beside=beside)
         self.step_graph = None    # H2D copies + search + D2H copies
         self.search_graph = None  # the search alone (inputs resident)
         # recorded after each step: load() waits for it before it overwrites
@@ -717,7 +720,8 @@ class PipelinedSession:
             per = periods if is_shared_grid(periods) else list(periods[a:b])
             dur = durations if is_shared_grid(durations) else list(durations[a:b])
             self.sessions.append(BatchSession(engine, pt[a:b + 1] - pt[a], per, dur, config,
-                                              y_dtype, weighted, fields))
+                                              y_dtype, weighted, fields,
+                                              len(self.streams)))
 
     @staticmethod
     def run_bounds(n_curves: int, parts: int) -> List[int]:

@@ -160,6 +160,14 @@ int atb_plan_create_async(atb_handle* h, const atb_params* params, const atb_bat
 int atb_plan_create_limited(atb_handle* h, const atb_params* params, const atb_batch* batch,
                             const atb_outputs* outputs, void* stream, int64_t table_bytes,
                             atb_plan** out);
+/*
+ * The plan of atb_plan_create for a caller that executes `beside` such plans at
+ * the same time, each on its own stream (no reference counterpart; results do not
+ * depend on it).  Steps that leave most of the GPU idle cost such a plan less,
+ * so it makes look-up tables for smaller batches.
+ */
+int atb_plan_create_beside(atb_handle* h, const atb_params* params, const atb_batch* batch,
+                           const atb_outputs* outputs, int32_t beside, atb_plan** out);
 int atb_plan_execute(atb_plan* p, void* stream);
 /* Synchronises `stream`-independent plan state: returns ATB_EDATA if the last
    execution met invalid input data, ATB_OK otherwise. */

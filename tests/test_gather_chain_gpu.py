@@ -3,6 +3,7 @@
 import numpy as np
 import pytest
 
+import recipes as R
 import test_gather_routes_gpu as G
 
 pytestmark = pytest.mark.gpu
@@ -65,3 +66,26 @@ def test_chained_kernels(engine, geom, wkind):
     del graphs
     for p in plans:
         p.close()
+
+
+def test_plans_that_run_beside_others_take_tables_earlier():
+    """Six curves are too few for tables when the GPU waits for them, not when it is shared."""
+    import torch
+    from astro_transit_gpu_b200.engine import BLSEngine, CurveBatch, SearchConfig
+    rng = np.random.default_rng(7)
+    n, nc = 34536, 6
+    t = [1000.0 + np.arange(n) * R.CADENCE_2MIN * 1.0001 for _ in range(nc)]
+    y = [(1.0 + rng.normal(0.0, 1e-3, n)).astype(np.float32) for _ in range(nc)]
+    batch = CurveBatch.from_arrays(t, y, periods=np.geomspace(0.78, 7.3, 6000),
+                                   durations=np.array([0.03, 0.08, 0.12, 0.16, 0.2]))
+    engine, cfg = BLSEngine.get(), SearchConfig("parity", objective="snr")
+    out = []
+    for beside in (1, 4):
+        plan = engine.plan(batch, cfg, beside=beside)
+        plan.execute()
+        plan.check()
+        out.append((plan.gathered()["counting"], plan.outputs))
+        plan.close()
+    assert out[0][0] == 0 and out[1][0] == nc * 6000
+    for k, v in out[0][1].items():
+        assert torch.equal(v, out[1][1][k]), k
